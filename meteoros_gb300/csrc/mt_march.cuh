@@ -195,17 +195,27 @@ MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, co
     const float* j = jitter[_index & 15];  // _index is in 0..15 for every finite t
     f3 jd = rc.dir + f3{j[0], j[1], j[2]};
     f3 pos = ld3(F.eye) + t * jd;
-    f3 sp = relative_position(F, pos, ld3(F.ec));
-    sp = rdiv3(sp, F.r_period);
-    float relH = relative_height(F, pos, ld3(F.ec), rc.lenInner, rc.dir, ld3(F.eye));
-    sp = sp + ((relH * ld3(F.skew)) * p.cloud_top_offset) * 0.009f;
-    sp = sp + ld3(F.wind_t);
+    const float relH = relative_height(F, pos, ld3(F.ec), rc.lenInner, rc.dir, ld3(F.eye));
+    // Empty steps, found before anything is fetched for them (results unchanged;
+    // of the benchmark views' executed steps 12 % are too high, 6 % have no
+    // gradient otherwise and 25 % only a gradient below the threshold.  960x540
+    // full frames 518 / 418 / 726 -> 504 / 385 / 690 us by view).  At heights from
+    // 0.65 both gradients are 0, whatever the cloud type ...
+    if (p.height_gradient && relH >= 0.65f) return o;
     Weather wt = weather_at<S>(p, F, tx, pos, ld3(F.ec));
     if (p.height_gradient) wt.hgrad = height_gradient(relH, wt.type);
-    // A zero height gradient or zero coverage makes the density 0 (or NaN
-    // when the coverage is 0), never > 0: the step is empty whatever the base
-    // volume holds, so its texture fetch is skipped (results unchanged).
+    // ... a zero height gradient or zero coverage makes the density 0 (or NaN
+    // when the coverage is 0), never > 0 ...
     if ((p.height_gradient && wt.hgrad == 0.0f) || wt.mul == 0.0f) return o;
+    // ... and so does a gradient that does not exceed the coverage threshold:
+    // the base shape is in [0, 1], so shape * gradient <= gradient <= lo (a
+    // product's rounding is monotone), the coverage remap clamps it to lo and
+    // its numerator lo - lo is 0 (0 / 0 = NaN when lo = 1, not > 0 either).
+    if (wt.hgrad <= wt.lo && wt.lo <= 1.0f) return o;
+    f3 sp = relative_position(F, pos, ld3(F.ec));
+    sp = rdiv3(sp, F.r_period);
+    sp = sp + ((relH * ld3(F.skew)) * p.cloud_top_offset) * 0.009f;
+    sp = sp + ld3(F.wind_t);
     float baseDensity = sample_low_frequency<S>(p, tx, sp, relH, wt) * 0.380f;
     if (baseDensity > 0.0f) {
         const Erosion ero = make_erosion(erosion_modifier<S>(tx, sp, relH));
