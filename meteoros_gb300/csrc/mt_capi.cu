@@ -240,7 +240,7 @@ mt_status build_march_args(mt_ctx* ctx, const mt_camera_ubo* cam, const mt_camer
     mt::make_view_consts(&a->vc_repro, *p, *cam, *cam_old, *tm, w, h, true);
     mt::make_view_consts(&a->vc_txaa, *p, *cam, *cam_old, *tm, w, h, false);
     mt::make_march_jitter(a->jitter, *tm);
-    mt::make_march_frame(&a->frame, *p, *cam, *tm);
+    mt::make_march_frame(&a->frame, *p, *cam, *tm, a->jitter);
     a->bottom_up = ctx->march_order == 0 ? 1 : 0;
     a->lanes = ctx->march_lanes;
     if (a->lanes == 0) {
@@ -731,7 +731,7 @@ MT_API mt_status mt_render_batch(mt_ctx* ctx, const mt_view* views, int n_views,
     mt_status st;
     if ((st = bind_device(ctx)) != MT_OK) return st;
     std::vector<mt::MarchArgs> args((size_t)n_views);
-    bool count = false;
+    bool count = false, tame = true;
     for (int i = 0; i < n_views; ++i) {
         const mt_view& v = views[i];
         st = build_march_args(ctx, &v.camera, &v.camera_old, &v.time, &v.params, v.prev_rgba, v.cur_rgba,
@@ -743,6 +743,7 @@ MT_API mt_status mt_render_batch(mt_ctx* ctx, const mt_view* views, int n_views,
         if (v.params.storage != views[0].params.storage)
             return fail(ctx, MT_ERR_INVALID_ARG, "view %d: all views of a batch must share one storage", i);
         count = count || (v.flags & MT_RENDER_COUNT);
+        tame = tame && args[(size_t)i].frame.tame;
         args[(size_t)i].bottom_up = ctx->batch_order == 0 ? 1 : 0;  // the order tile rows are handed out
     }
     // Tiles, most expensive views first (rays x steps), so the persistent
@@ -786,6 +787,7 @@ MT_API mt_status mt_render_batch(mt_ctx* ctx, const mt_view* views, int n_views,
     b.n_tiles = (int32_t)tiles.size();
     b.tile_w = tw;
     b.tile_h = th;
+    b.tame = tame ? 1 : 0;
     const int storage = views[0].params.storage;
     const int lanes = ctx->batch_lanes;
     int blocks = storage == MT_STORAGE_F16    ? mt::batch_blocks_f16(ctx->device, lanes)
@@ -1150,7 +1152,7 @@ MT_API mt_status mt_render_batch_noalloc(mt_ctx* ctx, const mt_view* views, int 
     mt::MarchArgs a;
     double cost[MT_NOALLOC_MAX_VIEWS];
     int nx[MT_NOALLOC_MAX_VIEWS], ny[MT_NOALLOC_MAX_VIEWS], bu[MT_NOALLOC_MAX_VIEWS], order[MT_NOALLOC_MAX_VIEWS];
-    bool count = false;
+    bool count = false, tame = true;
     for (int i = 0; i < n_views; ++i) {
         const mt_view& v = views[i];
         st = build_march_args(ctx, &v.camera, &v.camera_old, &v.time, &v.params, v.prev_rgba, v.cur_rgba,
@@ -1162,6 +1164,7 @@ MT_API mt_status mt_render_batch_noalloc(mt_ctx* ctx, const mt_view* views, int 
         if (v.params.storage != views[0].params.storage)
             return fail(ctx, MT_ERR_INVALID_ARG, "view %d: all views of a batch must share one storage", i);
         count = count || (v.flags & MT_RENDER_COUNT);
+        tame = tame && a.frame.tame;
         ray_grid(a, &nx[i], &ny[i]);
         bu[i] = ctx->batch_order == 0 ? 1 : 0;  // the order tile rows are handed out
         // most expensive views first, stable (mt_render_batch's order)
@@ -1225,6 +1228,7 @@ MT_API mt_status mt_render_batch_noalloc(mt_ctx* ctx, const mt_view* views, int 
     b.n_tiles = (int32_t)n_tiles;
     b.tile_w = tw;
     b.tile_h = th;
+    b.tame = tame ? 1 : 0;
     const int storage = views[0].params.storage;
     const int lanes = ctx->batch_lanes;
     const int blocks = storage == MT_STORAGE_F16    ? mt::batch_blocks_f16(ctx->device, lanes)

@@ -90,7 +90,44 @@ void make_march_jitter(float out[16][3], const mt_time_ubo& tm) {
     }
 }
 
-void make_march_frame(Frame* f, const mt_params& p, const mt_camera_ubo& cam, const mt_time_ubo& tm) {
+namespace {
+
+// Frame::tame.  The march divides by reused denominators with one Markstein
+// step (rdiv_core), exact unless a quotient overflows or is so small (below
+// 2^-100) that its residual underflows; rdiv checks for both.  Per step that
+// is six checks, a tenth of an empty step's instructions, and this settles
+// them once per frame (1080p frame 227 / 186 -> 221 / 182 us by view, 4K full
+// frames 5.36 / 3.55 -> 5.12 / 3.39 ms, 20-view batch 11.3 / 9.37 -> 10.9 / 8.97 ms):
+//   * no quotient is large: the scene's lengths are at most kFar, so positions
+//     (t at most the outer shell hit's distance, to the rounding of a quadratic
+//     in |eye| / radius) stay below 2^50 and quotients below 2^80;
+//   * a small quotient changes nothing.  Zero is exact up to its sign.  A
+//     texture coordinate below 2^-99 leaves s * N - 0.5 at -0.5.  The components
+//     of the up vector enter dot(dir, up) = (dx ux + dy uy) + dz uz, where dy is
+//     at least 0.06 (no other ray marches) and uy at least 2^-62 (the position's
+//     y stays half an Earth radius above the centre's: the eye's does, and dir.y
+//     + jitter.y is positive), so products below 2^-100 round away.  Heights'
+//     gradients and energies see 0 or differences of numbers near 1.
+// Other frames are marched with the checks (kGeneral).
+bool frame_is_tame(const Frame& f, const mt_params& p, const float jitter[16][3]) {
+    const double kFar = 0x1p30, kSmall = 0x1p-10, kScale = 0x1p-20;
+    auto len = [](const float v[3]) {
+        return std::sqrt((double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2]);
+    };
+    bool ok = len(f.eye) <= kFar && len(f.ec) <= kFar && f.Rout <= kFar && f.R >= kSmall && f.Rin >= kSmall &&
+              f.thickness >= kSmall && p.noise_period >= kScale && p.noise_period <= kFar &&
+              len(f.wind_t) <= kFar && len(f.skew) * std::fabs(p.cloud_top_offset) <= kFar &&
+              f.eye[1] >= -0.5f * f.R;
+    if (p.coverage_mode == 1) ok = ok && p.weather_scale >= kScale && p.weather_scale <= kFar;
+    for (int i = 0; i < 16; ++i)
+        for (int c = 0; c < 3; ++c) ok = ok && std::fabs(jitter[i][c]) <= 0.05f;
+    return ok;  // false for NaN
+}
+
+}  // namespace
+
+void make_march_frame(Frame* f, const mt_params& p, const mt_camera_ubo& cam, const mt_time_ubo& tm,
+                      const float jitter[16][3]) {
     f->R = p.earth_radius;
     f->Rin = p.shell_inner_radius;
     f->Rout = p.shell_outer_radius;
@@ -172,6 +209,7 @@ void make_march_frame(Frame* f, const mt_params& p, const mt_camera_ubo& cam, co
         const double* o = f->sh_o[s];
         f->sh_c[s] = (o[0] * o[0] + o[1] * o[1] + o[2] * o[2]) - 1.0;
     }
+    f->tame = frame_is_tame(*f, p, jitter) ? 1 : 0;
 }
 
 }  // namespace mt

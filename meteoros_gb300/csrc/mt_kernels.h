@@ -37,6 +37,8 @@ struct Rcp {
 // IEEE FP32 operations: kept in the kernel's parameter space, they take no
 // registers in the march loop.
 struct Frame {
+    // The march's per-step quotients need no range check (frame_is_tame)
+    int32_t tame;
     float R, Rin, Rout, thickness, inner_alt;  // earth radius, shell radii, Rout - Rin, Rin - R
     Rcp r_thick, r_period, r_weather;          // thickness, noise_period, weather_scale
     float eye[3];                              // ray origin: eye_sign * camera eye
@@ -61,7 +63,9 @@ struct Frame {
     float sky_betaR[3], sky_betaM[3], sky_betaRM[3];
 };
 
-void make_march_frame(Frame* f, const mt_params& p, const mt_camera_ubo& cam, const mt_time_ubo& tm);
+// `jitter`: the frame's step jitter (make_march_jitter)
+void make_march_frame(Frame* f, const mt_params& p, const mt_camera_ubo& cam, const mt_time_ubo& tm,
+                      const float jitter[16][3]);
 
 struct MarchArgs {
     mt_camera_ubo camera;
@@ -139,6 +143,7 @@ struct BatchArgs {
     unsigned long long* stats;  // or NULL
     int32_t n_tiles;
     int32_t tile_w, tile_h;     // tile shape in rays
+    int32_t tame;               // every view's frame is (Frame::tame)
 };
 
 // Outputs of one generator launch (any pointer may be NULL).

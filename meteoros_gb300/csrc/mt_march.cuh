@@ -59,7 +59,8 @@ template <int S> MT_HD Tex<S> make_tex(const MarchArgs& a) {
                   (const typename Vol<S>::T2*)a.vol[2], (const typename Vol<S>::T2*)a.vol[3]};
 }
 
-template <int S> MT_HD Weather weather_at(const mt_params& p, const Frame& F, const Tex<S>& tx, f3 pos, f3 ec) {
+template <int S, bool TAME>
+MT_HD Weather weather_at(const mt_params& p, const Frame& F, const Tex<S>& tx, f3 pos, f3 ec) {
     Weather w;
     w.hgrad = 1.0f;
     if (p.coverage_mode == 0) {
@@ -67,7 +68,7 @@ template <int S> MT_HD Weather weather_at(const mt_params& p, const Frame& F, co
         w.mul = p.coverage;
         w.type = 0.0f;
     } else {
-        const float2 wuv = rdiv2(pos.x - ec.x, pos.z - ec.z, F.r_weather);
+        const float2 wuv = rdiv2_step<TAME>(pos.x - ec.x, pos.z - ec.z, F.r_weather);
         f4v wd = Vol<S>::template tex2<MT_WEATHER_N>(tx.weather, wuv.x, wuv.y);
         w.lo = 1.0f - wd.x;
         w.mul = wd.x;
@@ -182,27 +183,34 @@ struct StepOut {
 };
 constexpr int kInCloud = 16;
 
+// How a march is compiled: for tame frames (Frame::tame: no range checks on the
+// steps' quotients), for every frame, and for every frame with the per-ray trace.
+constexpr int kTame = 0, kGeneral = 1, kTraced = 2;
+
 // One iteration of the march loop body (cloudRayMarch.comp:629-678) at
 // parameter t, up to the accumulation: everything that does not depend on the
 // running accumDensity / transmittance.
-template <int S, bool TR>
+template <int S, int MODE>
 MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, const mt_time_ubo& tm,
                         const float (*jitter)[3], const RayConsts& rc, float t) {
+    constexpr bool TAME = MODE == kTame, TR = MODE == kTraced;
     StepOut o{0, 0.0f, 0.0f};
     const int _index = f2i(gmod((float)(tm.frame_count_mod16 + f2i(t)), 16.0f));
     if (TR) o.code = _index & 15;
     const float* j = jitter[_index & 15];  // _index is in 0..15 for every finite t
     f3 jd = rc.dir + f3{j[0], j[1], j[2]};
     f3 pos = ld3(F.eye) + t * jd;
-    const float relH = relative_height(F, pos, ld3(F.ec), rc.lenInner, rc.dir, ld3(F.eye));
+    const float relH = relative_height<TAME>(F, pos, ld3(F.ec), rc.lenInner, rc.dir, ld3(F.eye));
     // Empty steps, found before anything is fetched for them (results unchanged;
     // of the benchmark views' executed steps 12 % are too high, 6 % have no
     // gradient otherwise and 25 % only a gradient below the threshold.  960x540
     // full frames 518 / 418 / 726 -> 504 / 385 / 690 us by view).  At heights from
     // 0.65 both gradients are 0, whatever the cloud type ...
     if (p.height_gradient && relH >= 0.65f) return o;
-    Weather wt = weather_at<S>(p, F, tx, pos, ld3(F.ec));
-    if (p.height_gradient) wt.hgrad = height_gradient(relH, wt.type);
+    Weather wt = weather_at<S, TAME>(p, F, tx, pos, ld3(F.ec));
+    // (the 16-bit forms keep its check: without it their compiler settings
+    // contract its blends another way, which moves their results by roundings)
+    if (p.height_gradient) wt.hgrad = height_gradient<TAME && S == MT_STORAGE_U8>(relH, wt.type);
     // ... a zero height gradient or zero coverage makes the density 0 (or NaN
     // when the coverage is 0), never > 0 ...
     if ((p.height_gradient && wt.hgrad == 0.0f) || wt.mul == 0.0f) return o;
@@ -211,8 +219,8 @@ MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, co
     // product's rounding is monotone), the coverage remap clamps it to lo and
     // its numerator lo - lo is 0 (0 / 0 = NaN when lo = 1, not > 0 either).
     if (wt.hgrad <= wt.lo && wt.lo <= 1.0f) return o;
-    f3 sp = relative_position(F, pos, ld3(F.ec));
-    sp = rdiv3(sp, F.r_period);
+    f3 sp = relative_position<TAME>(F, pos, ld3(F.ec));
+    sp = rdiv3_step<TAME>(sp, F.r_period);
     sp = sp + ((relH * ld3(F.skew)) * p.cloud_top_offset) * 0.009f;
     sp = sp + ld3(F.wind_t);
     float baseDensity = sample_low_frequency<S>(p, tx, sp, relH, wt) * 0.380f;
@@ -262,7 +270,7 @@ MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, co
                 }
             }
         }
-        o.E = light_energy(relH, dl, baseDensity, rc.HG_light, rc.cos_q, 5.0f);
+        o.E = light_energy<TAME>(relH, dl, baseDensity, rc.HG_light, rc.cos_q, 5.0f);
     }
     return o;
 }
@@ -274,7 +282,7 @@ MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, co
 // colour, the early exit) is then applied in step order by an in-group scan;
 // steps past the exit are discarded.  Result, counters and control flow equal
 // the sequential loop's.
-template <int G, int S, bool TR>
+template <int G, int S, int MODE>
 MT_HD f3 ray_march_group(const mt_params& p, const Frame& F, const Tex<S>& tx, const mt_time_ubo& tm,
                          const float (*jitter)[3], f3 dir, f3 startPos, float start_t, float end_t, float& accum,
                          Counts& cnt, unsigned gmask, int lane) {
@@ -302,7 +310,7 @@ MT_HD f3 ray_march_group(const mt_params& p, const Frame& F, const Tex<S>& tx, c
         for (int k = 0; k < lane; ++k) t += stepSize;
         const int valid = (t < end_t) && (s_base + lane < cap);
         StepOut o{0, 0.0f, 0.0f};
-        if (valid) o = eval_step<S, TR>(p, F, tx, tm, jitter, rc, t);
+        if (valid) o = eval_step<S, MODE>(p, F, tx, tm, jitter, rc, t);
 #pragma unroll
         for (int k = 0; k < G; ++k) {
             if (!__shfl_sync(gmask, valid, k, G)) {
@@ -313,7 +321,7 @@ MT_HD f3 ray_march_group(const mt_params& p, const Frame& F, const Tex<S>& tx, c
             const float hfd = __shfl_sync(gmask, o.hfd, k, G);
             const float E = __shfl_sync(gmask, o.E, k, G);
             if (lane == 0) cnt.primary++;
-            if (TR && lane == 0) cnt.sig = (cnt.sig ^ (unsigned)code) * 16777619u;  // FNV-1a step
+            if (MODE == kTraced && lane == 0) cnt.sig = (cnt.sig ^ (unsigned)code) * 16777619u;  // FNV-1a step
             if (code & kInCloud) {
                 accum = accum + hfd * 0.5f;
                 transmittance = gmix(transmittance, E, (1.0f - accum));
@@ -337,9 +345,10 @@ MT_HD f3 ray_march_group(const mt_params& p, const Frame& F, const Tex<S>& tx, c
 // cloudRayMarch.comp:690-826 for one pixel, marched by a group of G lanes;
 // lane 0 stores.  `jitter`: the view's per-step jitter table (a.jitter, or a
 // copy of it in shared memory).
-template <int G, int S, bool TR = false>
+template <int G, int S, int MODE>
 MT_HD void march_pixel(const MarchArgs& a, const Frame& F, const Tex<S>& tx, int px, int py, Counts& cnt,
                        unsigned gmask, int lane, const float (*jitter)[3]) {
+    constexpr bool TR = MODE == kTraced;
     const mt_params& p = a.params;
     const int W = a.width;
     // this frame's camera basis and cloudRayMarch.comp's jitter: the TXAA
@@ -386,7 +395,7 @@ MT_HD void march_pixel(const MarchArgs& a, const Frame& F, const Tex<S>& tx, int
     }
     float accum = 0.0f;
     if (TR) cnt.sig = 2166136261u;
-    f3 res = ray_march_group<G, S, TR>(p, F, tx, a.time, jitter, ray.direction, in.point, in.t, out.t, accum, cnt,
+    f3 res = ray_march_group<G, S, MODE>(p, F, tx, a.time, jitter, ray.direction, in.point, in.t, out.t, accum, cnt,
                                        gmask, lane);
     if (lane != 0) return;
     float godAccum = accum;
@@ -413,7 +422,7 @@ MT_HD void march_pixel(const MarchArgs& a, const Frame& F, const Tex<S>& tx, int
 constexpr int march_min_blocks(int G, int BS) {
     return ((G == 1 ? 1280 : 1024) / BS) < 32 ? ((G == 1 ? 1280 : 1024) / BS) : 32;  // at most 32 CTAs an SM
 }
-template <int G, int S, int BS, bool TR = false>
+template <int G, int S, int BS, int MODE>
 __global__ void __launch_bounds__(BS, march_min_blocks(G, BS)) march_kernel(const __grid_constant__ MarchArgs a) {
     static_assert(G >= 1 && G <= 32 && (32 % G) == 0, "G must divide the warp");
     const Frame& F = a.frame;
@@ -445,7 +454,7 @@ __global__ void __launch_bounds__(BS, march_min_blocks(G, BS)) march_kernel(cons
         }
     }
     if (active) {
-        march_pixel<G, S, TR>(a, F, tx, px, py, cnt, gmask, lane, s_jitter);
+        march_pixel<G, S, MODE>(a, F, tx, px, py, cnt, gmask, lane, s_jitter);
         pixels = lane == 0 ? 1u : 0u;
     }
     if (a.stats) flush_counts(a.stats, cnt, pixels);
@@ -457,7 +466,7 @@ __global__ void __launch_bounds__(BS, march_min_blocks(G, BS)) march_kernel(cons
 // marches its rays, 128/G rays per pass; per-view arguments come from the
 // view table in global memory.  Per-pixel results equal those of separate
 // march_kernel launches (the same march_pixel runs on the same inputs).
-template <int G, int S>
+template <int G, int S, int MODE>
 __global__ void __launch_bounds__(128, 8) march_batch_kernel(const __grid_constant__ BatchArgs b) {
     __shared__ int s_tile;
     const int lane = (int)(threadIdx.x % G);
@@ -486,7 +495,7 @@ __global__ void __launch_bounds__(128, 8) march_batch_kernel(const __grid_consta
             const int px = rx * step + sx, py = ry * step + sy;
             const bool active = r < tile_rays && rx < tile.nrx && ry < tile.nry && px < a.width && py < a.height;
             if (active) {
-                march_pixel<G, S>(a, F, tx, px, py, cnt, gmask, lane, a.jitter);
+                march_pixel<G, S, MODE>(a, F, tx, px, py, cnt, gmask, lane, a.jitter);
                 pixels += lane == 0 ? 1u : 0u;
             }
         }
@@ -495,11 +504,15 @@ __global__ void __launch_bounds__(128, 8) march_batch_kernel(const __grid_consta
 }
 
 template <int S> cudaError_t launch_batch_storage(const BatchArgs& b, int lanes, int blocks, cudaStream_t s) {
+    if (!b.tame) {
+        march_batch_kernel<1, S, kGeneral><<<blocks, 128, 0, s>>>(b);
+        return cudaGetLastError();
+    }
     switch (lanes) {
-        case 1: march_batch_kernel<1, S><<<blocks, 128, 0, s>>>(b); break;
-        case 4: march_batch_kernel<4, S><<<blocks, 128, 0, s>>>(b); break;
-        case 16: march_batch_kernel<16, S><<<blocks, 128, 0, s>>>(b); break;
-        default: march_batch_kernel<8, S><<<blocks, 128, 0, s>>>(b); break;
+        case 1: march_batch_kernel<1, S, kTame><<<blocks, 128, 0, s>>>(b); break;
+        case 4: march_batch_kernel<4, S, kTame><<<blocks, 128, 0, s>>>(b); break;
+        case 16: march_batch_kernel<16, S, kTame><<<blocks, 128, 0, s>>>(b); break;
+        default: march_batch_kernel<8, S, kTame><<<blocks, 128, 0, s>>>(b); break;
     }
     return cudaGetLastError();
 }
@@ -507,11 +520,12 @@ template <int S> cudaError_t launch_batch_storage(const BatchArgs& b, int lanes,
 template <int S> int batch_blocks_storage(int device, int lanes) {
     int per_sm = 0, sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    auto occupancy = [&](auto kernel) { cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0); };
     switch (lanes) {
-        case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_batch_kernel<1, S>, 128, 0); break;
-        case 4: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_batch_kernel<4, S>, 128, 0); break;
-        case 16: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_batch_kernel<16, S>, 128, 0); break;
-        default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_batch_kernel<8, S>, 128, 0); break;
+        case 1: occupancy(march_batch_kernel<1, S, kTame>); break;
+        case 4: occupancy(march_batch_kernel<4, S, kTame>); break;
+        case 16: occupancy(march_batch_kernel<16, S, kTame>); break;
+        default: occupancy(march_batch_kernel<8, S, kTame>); break;
     }
     return (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
 }
@@ -520,21 +534,28 @@ template <int S, int BS> void launch_march_bs(const MarchArgs& a, cudaStream_t s
     const int G = a.lanes;
     const unsigned blocks = (unsigned)((rays * G + BS - 1) / BS);
     switch (G) {
-        case 1: march_kernel<1, S, BS><<<blocks, BS, 0, s>>>(a); break;
-        case 4: march_kernel<4, S, BS><<<blocks, BS, 0, s>>>(a); break;
-        case 16: march_kernel<16, S, BS><<<blocks, BS, 0, s>>>(a); break;
-        default: march_kernel<8, S, BS><<<blocks, BS, 0, s>>>(a); break;
+        case 1: march_kernel<1, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
+        case 4: march_kernel<4, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
+        case 16: march_kernel<16, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
+        default: march_kernel<8, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
     }
 }
 
 template <int S> cudaError_t launch_march_storage(const MarchArgs& a, cudaStream_t s, long long rays) {
-    if (a.trace) {  // traced march (mt_set_sample_trace): 256-thread CTAs, 1 or 4 lanes
+    if (a.trace || !a.frame.tame) {  // 256-thread CTAs, 1 or 4 lanes
         const int G = a.lanes == 1 ? 1 : 4;
         const unsigned blocks = (unsigned)((rays * G + 255) / 256);
-        if (G == 1)
-            march_kernel<1, S, 256, true><<<blocks, 256, 0, s>>>(a);
-        else
-            march_kernel<4, S, 256, true><<<blocks, 256, 0, s>>>(a);
+        if (a.trace) {
+            if (G == 1)
+                march_kernel<1, S, 256, kTraced><<<blocks, 256, 0, s>>>(a);
+            else
+                march_kernel<4, S, 256, kTraced><<<blocks, 256, 0, s>>>(a);
+        } else {
+            if (G == 1)
+                march_kernel<1, S, 256, kGeneral><<<blocks, 256, 0, s>>>(a);
+            else
+                march_kernel<4, S, 256, kGeneral><<<blocks, 256, 0, s>>>(a);
+        }
         return cudaGetLastError();
     }
     if (a.block == 256)

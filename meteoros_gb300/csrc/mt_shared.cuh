@@ -11,8 +11,8 @@ namespace mt {
 
 // remap() whose range width omax - omin is known ahead: the quotient through
 // the correctly rounded reciprocal of that width (rdiv).
-MT_HD float remap_r(float v, float omin, Rcp width, float nmin, float nmax) {
-    return nmin + ((rdiv(v - omin, width)) * (nmax - nmin));
+template <bool TAME> MT_HD float remap_r(float v, float omin, Rcp width, float nmin, float nmax) {
+    return nmin + ((rdiv_step<TAME>(v - omin, width)) * (nmax - nmin));
 }
 // The reciprocal of a compile-time width, rounded once by the compiler.
 #define MT_RCP(omin, omax) (Rcp{(omax) - (omin), 1.0f / ((omax) - (omin))})
@@ -117,17 +117,19 @@ MT_HD float remap_clamped(float v, float omin, float omax, float nmin, float nma
 // cloudRayMarch.comp:171-186
 // lenInner = length(startPos - eye) is the same for every step of a ray; the
 // raymarch passes it in precomputed.
+template <bool TAME>
 MT_HD float relative_height(const Frame& F, f3 point, f3 ec, float lenInner, f3 rayDir, f3 eye) {
     float lenCam = length3(point - eye);
-    f3 p2e = normalize3_r(point - ec);
+    const f3 up = point - ec;
+    f3 p2e = rdiv3_step<TAME>(up, make_rcp(length3(up)));
     float cosTheta = dot3(rayDir, p2e);
     float num = fabsf(cosTheta * (lenCam - lenInner));
-    return rdiv(num, F.r_thick);
+    return rdiv_step<TAME>(num, F.r_thick);
 }
 
 // cloudRayMarch.comp:188-191
-MT_HD f3 relative_position(const Frame& F, f3 pos, f3 ec) {
-    return rdiv3(pos - f3{ec.x, F.inner_alt, ec.z}, F.r_thick);
+template <bool TAME> MT_HD f3 relative_position(const Frame& F, f3 pos, f3 ec) {
+    return rdiv3_step<TAME>(pos - f3{ec.x, F.inner_alt, ec.z}, F.r_thick);
 }
 
 // The four quotients of height_gradient's remaps, (h - omin) / (omax - omin).
@@ -141,11 +143,11 @@ static __device__ __noinline__ HgQuot hg_quotients_exceptional(float h) {
 
 // cloudRayMarch.comp:475-487.  The remaps' four quotients share one range
 // check (rdiv_core; all four redone by rdiv when any falls outside it).
-MT_HD float height_gradient(float h, float type) {
+template <bool TAME> MT_HD float height_gradient(float h, float type) {
     h = gclamp(h, 0.0f, 1.0f);
     HgQuot q{rdiv_core(h - 0.0f, MT_RCP(0.0f, 0.25f)), rdiv_core(h - 0.3f, MT_RCP(0.3f, 0.65f)),
              rdiv_core(h - 0.0f, MT_RCP(0.0f, 0.1f)), rdiv_core(h - 0.2f, MT_RCP(0.2f, 0.3f))};
-    if (!(rdiv_in_range(q.q1) & rdiv_in_range(q.q2) & rdiv_in_range(q.q3) & rdiv_in_range(q.q4)))
+    if (!TAME && !(rdiv_in_range(q.q1) & rdiv_in_range(q.q2) & rdiv_in_range(q.q3) & rdiv_in_range(q.q4)))
         q = hg_quotients_exceptional(h);
     // remap(h, omin, omax, nmin, nmax) = nmin + q * (nmax - nmin)
     float stratocumulus = gmax(0.0f, (0.0f + (q.q1 * (1.0f - 0.0f))) * (1.0f + (q.q2 * (0.0f - 1.0f))));
@@ -183,12 +185,12 @@ MT_HD float henyey_greenstein(float c, float e) {
 // which is how GLSL defines pow's precision: they differ from the correctly
 // rounded values by tens of ulp at most.  The light energy reaches colour
 // only, never the accumulated density, the control flow or the god-ray mask.
-MT_HD float light_energy(float h, float dl, float ds, float phase, float cos_q, float brightness) {
+template <bool TAME> MT_HD float light_energy(float h, float dl, float ds, float phase, float cos_q, float brightness) {
     const float primary = __expf(-dl);
     const float secondary = primary;  // exp(-dl) twice in the reference (:334, :340)
     float att = gmax(secondary + (cos_q * (secondary * 0.25f - secondary)), primary);
-    float depth = 0.05f + __powf(ds, gclamp(remap_r(h * 0.125f, 0.3f, MT_RCP(0.3f, 0.85f), 0.5f, 2.0f), 0.5f, 2.0f));
-    float vert = __powf(gclamp(remap_r(h * 1.5f, 0.07f, MT_RCP(0.07f, 0.34f), 0.1f, 1.0f), 0.1f, 1.0f), 0.8f);
+    float depth = 0.05f + __powf(ds, gclamp(remap_r<TAME>(h * 0.125f, 0.3f, MT_RCP(0.3f, 0.85f), 0.5f, 2.0f), 0.5f, 2.0f));
+    float vert = __powf(gclamp(remap_r<TAME>(h * 1.5f, 0.07f, MT_RCP(0.07f, 0.34f), 0.1f, 1.0f), 0.1f, 1.0f), 0.8f);
     float in_scatter = depth * vert;
     return att * primary * in_scatter * phase * brightness;
 }

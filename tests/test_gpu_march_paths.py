@@ -58,3 +58,67 @@ def test_empty_step_rules_weather_extremes(ctx, oracle, volumes_seed7, kind):
     cam, tm, params, _ = scenes.config_view(4, W, H)
     params.weather_slot = 9
     check_density(oracle, vol, ctx, params, cam, tm)
+
+
+@pytest.fixture(scope="module")
+def trace_buffer():
+    return torch.zeros((H, W, 4), dtype=torch.int32, device="cuda")
+
+
+def scene(name):
+    cam, tm, params, _ = scenes.config_view(3, W, H)
+    if name == "reference":
+        cam, tm, params = scenes.reference_frame(W, H, 9.0, 3, 1.0)
+    elif name == "axis":  # rays in the x = 0 plane: quotients of exact zeros
+        cam = scenes.look((0.0, 100.0, 0.0), 0.0, 20.0, 60.0, W, H)
+        for seq in (tm.halton_seq1, tm.halton_seq2, tm.halton_seq3, tm.halton_seq4):
+            seq[:] = [0.0] * 4
+    elif name == "far eye":  # just inside the bound on lengths, and beyond it
+        cam.eye[0], cam.eye[2] = 0.9e9, 0.3e9
+    elif name == "beyond":
+        cam.eye[0] = 4.0e9
+    elif name == "small scales":
+        params.noise_period, params.weather_scale = 2.0 ** -19, 2.0 ** -19
+    elif name == "still air":
+        params.wind_speed, params.cloud_top_offset = 0.0, 0.0
+    elif name == "storm":  # beyond the bound on the wind's offset
+        params.wind_speed, tm.time[1] = 1.0e9, 1.0e3
+    elif name == "jitter":  # beyond the bound on the steps' jitter
+        tm.halton_seq1[0], tm.halton_seq2[1] = 6.0, -6.0
+    return cam, tm, params
+
+
+SCENES = ["config", "reference", "axis", "far eye", "beyond", "small scales", "still air", "storm", "jitter"]
+
+
+@pytest.mark.parametrize("storage", [abi.MT_STORAGE_U8, abi.MT_STORAGE_F16, abi.MT_STORAGE_BF16])
+@pytest.mark.parametrize("name", SCENES)
+def test_unchecked_quotients_equal_checked(ctx, trace_buffer, name, storage):
+    """Frames whose scene bounds every quotient march without range checks;
+    a traced render always checks.  Both give the same bits, on either side
+    of the bounds, one view at a time and in a batch."""
+    cam, tm, params = scene(name)
+    params.storage, params.fp64_shells = storage, int(storage != abi.MT_STORAGE_U8)
+    frames = []
+    for lanes, traced in ((1, True), (1, False), (4, True), (4, False)):
+        cur = torch.full((H, W, 4), float("nan"), device="cuda")
+        mask = torch.full((H, W), float("nan"), device="cuda")
+        ctx.set_tuning(march_lanes=lanes)
+        ctx.set_sample_trace(trace_buffer if traced else None)
+        ctx.render(cam, cam, tm, params, None, cur, mask, abi.MT_RENDER_FULL)
+        frames.append((cur, mask))
+    ctx.set_sample_trace(None)
+    ctx.set_tuning(march_lanes=0)
+    cur, mask = torch.zeros((H, W, 4), device="cuda"), torch.zeros((H, W), device="cuda")
+    ctx.render_batch([scenes.make_view(cam, cam, tm, params, cur, None, mask, abi.MT_RENDER_FULL)])
+    frames.append((cur, mask))
+    torch.cuda.synchronize()
+    for cur, mask in frames[1:]:
+        assert_bits_equal(cur.cpu().numpy(), frames[0][0].cpu().numpy(), name)
+        assert_bits_equal(mask.cpu().numpy(), frames[0][1].cpu().numpy(), name)
+
+
+@pytest.mark.parametrize("name", ["axis", "still air", "small scales", "jitter"])
+def test_quotient_edges_equal_oracle(ctx, oracle, vol7, name):
+    cam, tm, params = scene(name)
+    check_density(oracle, vol7, ctx, params, cam, tm)
