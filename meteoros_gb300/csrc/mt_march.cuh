@@ -281,7 +281,13 @@ MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, co
 // bit-identical t.  The loop-carried part (accumDensity, transmittance,
 // colour, the early exit) is then applied in step order by an in-group scan;
 // steps past the exit are discarded.  Result, counters and control flow equal
-// the sequential loop's.
+// the sequential loop's.  Three forms of the scan: one lane applies its own step
+// (a scan over one lane still shuffled five times a step: 4K full frames 5.04 /
+// 3.34 -> 4.69 / 3.16 ms by view, FP16 4.74 / 3.11 -> 4.12 / 2.81, 20-view batch
+// 10.8 / 8.89 -> 9.85 / 8.28 ms); 2 and 4 lanes take the steps one by one,
+// unrolled; longer groups loop over the in-cloud steps (640x360 frames at 16
+// lanes 59.5 / 55.7 -> 52.6 / 45.1 us; at 4 lanes 219 -> 223 us for the 1080p
+// frame, so not there).
 template <int G, int S, int MODE>
 MT_HD f3 ray_march_group(const mt_params& p, const Frame& F, const Tex<S>& tx, const mt_time_ubo& tm,
                          const float (*jitter)[3], f3 dir, f3 startPos, float start_t, float end_t, float& accum,
@@ -302,6 +308,8 @@ MT_HD f3 ray_march_group(const mt_params& p, const Frame& F, const Tex<S>& tx, c
     // never advance.  A valid ray runs steps or steps+1 iterations.
     const int cap = 2 * f2i(maxSteps) + 8;
     if (lane == 0) cnt.rays++;
+    constexpr unsigned kGroup = G == 32 ? 0xffffffffu : (1u << G) - 1u;
+    const int shift = (int)(threadIdx.x & 31u) & ~(G - 1);  // the group's first lane
     float t_base = start_t;
     int s_base = 0;
     bool done = false;
@@ -311,30 +319,73 @@ MT_HD f3 ray_march_group(const mt_params& p, const Frame& F, const Tex<S>& tx, c
         const int valid = (t < end_t) && (s_base + lane < cap);
         StepOut o{0, 0.0f, 0.0f};
         if (valid) o = eval_step<S, MODE>(p, F, tx, tm, jitter, rc, t);
-#pragma unroll
-        for (int k = 0; k < G; ++k) {
-            if (!__shfl_sync(gmask, valid, k, G)) {
-                done = true;
-                break;
-            }
-            const int code = __shfl_sync(gmask, o.code, k, G);
-            const float hfd = __shfl_sync(gmask, o.hfd, k, G);
-            const float E = __shfl_sync(gmask, o.E, k, G);
-            if (lane == 0) cnt.primary++;
-            if (MODE == kTraced && lane == 0) cnt.sig = (cnt.sig ^ (unsigned)code) * 16777619u;  // FNV-1a step
-            if (code & kInCloud) {
-                accum = accum + hfd * 0.5f;
-                transmittance = gmix(transmittance, E, (1.0f - accum));
-                color = color + f3{transmittance, transmittance, transmittance};
-                if (lane == 0) cnt.light += 6;
-            }
+        auto apply = [&](float hfd, float E) {
+            accum = accum + hfd * 0.5f;
+            const float k = 1.0f - accum;
+            // mix(transmittance, E, k); the 16-bit forms' compiler settings would
+            // contract it, so they state their contraction
+            transmittance = S == MT_STORAGE_U8 ? gmix(transmittance, E, k)
+                                               : __fmaf_rn(E, k, __fmul_rn(transmittance, 1.0f - k));
+            color = color + f3{transmittance, transmittance, transmittance};
+            if (lane == 0) cnt.light += 6;
+        };
+        if constexpr (G == 1) {
+            if (!valid) break;
+            cnt.primary++;
+            if (MODE == kTraced) cnt.sig = (cnt.sig ^ (unsigned)o.code) * 16777619u;  // FNV-1a step
+            if (o.code & kInCloud) apply(o.hfd, o.E);
             if (accum >= p.accum_limit) {
                 accum = 1.0f;
-                done = true;
                 break;
             }
+            t_base = t + stepSize;
+            s_base++;
+        } else if constexpr (G <= 4) {
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+                if (!__shfl_sync(gmask, valid, k, G)) {
+                    done = true;
+                    break;
+                }
+                const int code = __shfl_sync(gmask, o.code, k, G);
+                const float hfd = __shfl_sync(gmask, o.hfd, k, G);
+                const float E = __shfl_sync(gmask, o.E, k, G);
+                if (lane == 0) cnt.primary++;
+                if (MODE == kTraced && lane == 0) cnt.sig = (cnt.sig ^ (unsigned)code) * 16777619u;
+                if (code & kInCloud) apply(hfd, E);
+                if (accum >= p.accum_limit) {
+                    accum = 1.0f;
+                    done = true;
+                    break;
+                }
+            }
+        } else {
+            // Only in-cloud steps move the accumulated density, so only after
+            // them can the ray end early (and after its first step, should the
+            // limit not lie above 0): a loop over those, where the steps of a
+            // long chunk one by one take four shuffles each.
+            static_assert(G <= 4 || MODE != kTraced, "traced marches use 1 or 4 lanes");
+            const unsigned in_chunk = __ballot_sync(gmask, valid) >> shift & kGroup;  // the first steps
+            const unsigned cloud = __ballot_sync(gmask, (o.code & kInCloud) != 0) >> shift & kGroup;
+            int executed = __popc(in_chunk);
+            done = executed < G;
+            unsigned events = (cloud | (accum >= p.accum_limit ? 1u : 0u)) & in_chunk;
+            while (events) {
+                const int k = __ffs((int)events) - 1;
+                events &= events - 1u;
+                const float hfd = __shfl_sync(gmask, o.hfd, k, G);
+                const float E = __shfl_sync(gmask, o.E, k, G);
+                if (cloud >> k & 1u) apply(hfd, E);
+                if (accum >= p.accum_limit) {
+                    accum = 1.0f;
+                    done = true;
+                    executed = k + 1;
+                    break;
+                }
+            }
+            if (lane == 0) cnt.primary += executed;
         }
-        if (!done) {
+        if (G > 1 && !done) {
             t_base = __shfl_sync(gmask, t, G - 1, G) + stepSize;
             s_base += G;
         }
@@ -411,19 +462,21 @@ MT_HD void march_pixel(const MarchArgs& a, const Frame& F, const Tex<S>& tx, int
 // groups_x x groups_y blocks of 4x4 (Renderer.cpp:713-716); each ray is one
 // block's slot pixel.  Full: one ray per pixel.  G consecutive lanes (an
 // aligned segment of a warp) march one ray.  BS threads per CTA (256 by
-// default, 128 or 32 selectable).  Resident threads per SM: 1024 (64
-// registers a thread) when G lanes share a ray; 1280 (48 registers, a few
-// spills) for one lane per ray, whose full-frame launches run 2-3 % faster
-// for the extra warps while the 4-lane checkerboard launches gain nothing.
+// default, 128 or 32 selectable).  Resident threads per SM: 1024 (64 registers
+// a thread), or for one lane per ray on FP16 volumes 1280 (48, with some 200 B
+// of spills: 4K 4.12 ms for 4.19; RGBA8 took 4.69 ms so for 4.62, and bfloat16
+// 1603x901 1.06 ms for 1.01).
 // Every step reads its jitter vector at an index taken from int(t), which
 // differs from lane to lane: from the parameter space a warp's reads at up to
 // 16 different words are served one word at a time, from shared memory in one
 // pass (48 words, 3 apart: distinct banks), so the table is copied there.
-constexpr int march_min_blocks(int G, int BS) {
-    return ((G == 1 ? 1280 : 1024) / BS) < 32 ? ((G == 1 ? 1280 : 1024) / BS) : 32;  // at most 32 CTAs an SM
+constexpr int march_min_blocks(int G, int S, int BS) {
+    const int n = (G == 1 && S == MT_STORAGE_F16 ? 1280 : 1024) / BS;
+    return n < 32 ? n : 32;  // at most 32 CTAs an SM
 }
 template <int G, int S, int BS, int MODE>
-__global__ void __launch_bounds__(BS, march_min_blocks(G, BS)) march_kernel(const __grid_constant__ MarchArgs a) {
+__global__ void __launch_bounds__(BS, march_min_blocks(G, S, BS))
+    march_kernel(const __grid_constant__ MarchArgs a) {
     static_assert(G >= 1 && G <= 32 && (32 % G) == 0, "G must divide the warp");
     const Frame& F = a.frame;
     const Tex<S> tx = make_tex<S>(a);

@@ -122,3 +122,14 @@ def test_unchecked_quotients_equal_checked(ctx, trace_buffer, name, storage):
 def test_quotient_edges_equal_oracle(ctx, oracle, vol7, name):
     cam, tm, params = scene(name)
     check_density(oracle, vol7, ctx, params, cam, tm)
+
+
+@pytest.mark.parametrize("limit", [0.99, 0.3, 0.0, -1.0])
+@pytest.mark.parametrize("lanes", [0, 1, 4, 8, 16])
+def test_early_exit_at_every_limit(ctx, oracle, vol7, lanes, limit):
+    """A limit at or below 0 ends a ray after its first step, in cloud or not."""
+    cam, tm, params, _ = scenes.config_view(3, W, H)
+    params.accum_limit = limit
+    ctx.set_tuning(march_lanes=lanes)
+    check_density(oracle, vol7, ctx, params, cam, tm)
+    ctx.set_tuning(march_lanes=0)
