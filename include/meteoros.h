@@ -155,7 +155,8 @@ typedef struct mt_kernel_times {
 /* Launch-shape choices of the kernels.  Results do not depend on them (the
  * tests hold every choice to the same output); only speed does. */
 typedef struct mt_tuning {
-    int32_t march_lanes;  /* lanes that march one ray together: 1, 4, 8 or 16; 0 = chosen from the ray count */
+    int32_t march_lanes;  /* lanes that march one ray together: 1, 4, 8 or 16; 0 = chosen from the ray
+                           * count (1, 2, 4, 8, 16 or 32) */
     int32_t fused_resolve; /* mt_render_frame: 0 = the raymarch, the TXAA history taps and the
                             * reprojection in one kernel beside it, then the TXAA resolve (default);
                             * 1 = the raymarch, then the reprojection fused with the TXAA resolve */

@@ -243,12 +243,8 @@ mt_status build_march_args(mt_ctx* ctx, const mt_camera_ubo* cam, const mt_camer
     mt::make_march_frame(&a->frame, *p, *cam, *tm, a->jitter);
     a->bottom_up = ctx->march_order == 0 ? 1 : 0;
     a->lanes = ctx->march_lanes;
-    if (a->lanes == 0) {
-        // Auto: enough rays fill the GPU one lane per ray; fewer rays (a
-        // checkerboard frame marches 1/16 of the pixels) get 4 lanes each.
-        const long long rays = full ? (long long)w * h : (long long)a->groups_x * a->groups_y;
-        a->lanes = rays >= 262144 ? 1 : 4;
-    }
+    // (a checkerboard frame marches a sixteenth of its pixels)
+    if (a->lanes == 0) a->lanes = mt::auto_lanes((long long)w * h / (full ? 1 : 16));
     return MT_OK;
 }
 

@@ -86,7 +86,7 @@ struct MarchArgs {
     int32_t width, height;
     int32_t groups_x, groups_y;  // 4x4 blocks covered by the reference's raymarch dispatch
     uint32_t flags;
-    int32_t lanes;               // lanes marching one ray together: 1, 4, 8 or 16
+    int32_t lanes;               // lanes marching one ray together: 1, 2, 4, 8, 16 or 32
     int32_t block;               // march_kernel CTA size: 32, 128 or 256 threads
     // Dispatch order of the ray rows (rows of 4x4 blocks, or of pixels for a
     // full frame): 1 = bottom to top (default), 0 = top to bottom.  Bottom to
@@ -109,6 +109,25 @@ struct MarchArgs {
     float jitter[16][3];
     Frame frame;
 };
+
+// Lanes that march one ray together when the tuning leaves it open, by the rays
+// of the launch.  More lanes shorten a ray's serial chain (alone some 220 us at
+// one lane, 25 at 32) and fill the 152 SMs' 155 648 resident threads; they also
+// compute steps past a ray's exit and scan.  Measured both sides of each line,
+// us by view (frames are checkerboard, 1/16 of the pixels):
+//   32 | 16  480x270 frame 48 / 36 | 44 / 42, 128x72 full 37 / 26 | 31 / 31
+//   16 | 8   800x450 frame 67 / 54 | 72 / 68, 960x540 frame 86 / 69 | 79 / 73
+//   8 | 4    1440x810 frame 147 / 123 | 142 / 161, 1600x900 frame 177 / 149 | 165 / 160
+//   4 | 2    2240x1260 frame 295 / 243 | 276 / 288, 2560x1440 frame 375 / 309 | 344 / 291
+//   2 | 1    3000x1688 frame 467 / 389 | 481 / 463, 960x540 full 410 / 259 | 410 / 255,
+//            3840x2160 frame 737 / 615 | 700 / 586
+inline int auto_lanes(long long rays) {
+    if (rays <= 8192) return 32;
+    if (rays <= 28000) return 16;
+    if (rays <= 90000) return 8;
+    if (rays <= 210000) return 4;
+    return rays <= 450000 ? 2 : 1;
+}
 
 void make_march_jitter(float out[16][3], const mt_time_ubo& tm);
 

@@ -588,6 +588,8 @@ template <int S, int BS> void launch_march_bs(const MarchArgs& a, cudaStream_t s
     const unsigned blocks = (unsigned)((rays * G + BS - 1) / BS);
     switch (G) {
         case 1: march_kernel<1, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
+        case 2: march_kernel<2, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
+        case 32: march_kernel<32, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
         case 4: march_kernel<4, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
         case 16: march_kernel<16, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
         default: march_kernel<8, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;

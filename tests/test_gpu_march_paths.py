@@ -124,6 +124,25 @@ def test_quotient_edges_equal_oracle(ctx, oracle, vol7, name):
     check_density(oracle, vol7, ctx, params, cam, tm)
 
 
+@pytest.mark.parametrize("size", [(16, 8), (90, 91), (91, 91), (167, 168), (300, 300), (300, 301), (458, 459), (670, 672),
+                                  (671, 671)])
+def test_lane_counts_by_size_give_one_frame(ctx, size):
+    """The lanes per ray follow the ray count; each line's two sides, marched
+    as chosen and at one lane, counters included."""
+    w, h = size
+    cam, tm, params, _ = scenes.config_view(5, w, h)
+    frames = []
+    for lanes in (0, 1):
+        ctx.set_tuning(march_lanes=lanes)
+        frames.append(gpu_render(ctx, cam, cam, tm, params, None, w, h, abi.MT_RENDER_FULL))
+    ctx.set_tuning(march_lanes=0)
+    (a, am, sa), (b, bm, sb) = frames
+    assert_bits_equal(a, b, "rgba")
+    assert_bits_equal(am, bm, "mask")
+    assert (sa.primary_samples, sa.light_samples, sa.marched_rays, sa.pixels) == \
+        (sb.primary_samples, sb.light_samples, sb.marched_rays, sb.pixels)
+
+
 @pytest.mark.parametrize("limit", [0.99, 0.3, 0.0, -1.0])
 @pytest.mark.parametrize("lanes", [0, 1, 4, 8, 16])
 def test_early_exit_at_every_limit(ctx, oracle, vol7, lanes, limit):
