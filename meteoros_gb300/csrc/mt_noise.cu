@@ -11,7 +11,8 @@
 // -fmad=false), so the output is bit-identical to the CPU generator that the
 // tests hold it against.
 //
-// One thread per texel.  Outputs: RGBA8 words plus IEEE half and bfloat16
+// One thread per texel; the base volume, 27 cells in each of nine Worley
+// octaves a texel, takes 2x2x2 texels a thread.  Outputs: RGBA8 words plus IEEE half and bfloat16
 // copies for the precision form, all in create3DTextureFromMany2DTextures
 // layout (x fastest, then y, then slice z).
 #include <cuda_bf16.h>
@@ -73,57 +74,6 @@ __device__ float worley3(float px, float py, float pz, int F, uint32_t s) {
     return 1.0f - (d < 1.0f ? d : 1.0f);
 }
 
-__device__ float worley_fbm3(float x, float y, float z, int F, uint32_t s) {
-    float f0 = (float)F, f1 = (float)(2 * F), f2 = (float)(4 * F);
-    float w0 = worley3(x * f0, y * f0, z * f0, F, s);
-    float w1 = worley3(x * f1, y * f1, z * f1, 2 * F, s + 1u);
-    float w2 = worley3(x * f2, y * f2, z * f2, 4 * F, s + 2u);
-    return (w0 * 0.625f + w1 * 0.25f) + w2 * 0.125f;
-}
-
-__device__ __forceinline__ float grad3(uint32_t h, float x, float y, float z) {
-    h &= 15u;
-    float u = h < 8u ? x : y;
-    float v = h < 4u ? y : ((h == 12u || h == 14u) ? x : z);
-    return ((h & 1u) ? -u : u) + ((h & 2u) ? -v : v);
-}
-
-__device__ float perlin3(float px, float py, float pz, int F, uint32_t s) {
-    const uint32_t m = (uint32_t)F - 1u;
-    float fx = floorf(px), fy = floorf(py), fz = floorf(pz);
-    int ix = (int)fx, iy = (int)fy, iz = (int)fz;
-    float x = px - fx, y = py - fy, z = pz - fz;
-    float u = fade(x), v = fade(y), w = fade(z);
-    uint32_t x0 = (uint32_t)ix & m, x1 = (uint32_t)(ix + 1) & m;
-    uint32_t y0 = (uint32_t)iy & m, y1 = (uint32_t)(iy + 1) & m;
-    uint32_t z0 = (uint32_t)iz & m, z1 = (uint32_t)(iz + 1) & m;
-    float g000 = grad3(hash3(x0, y0, z0, s), x, y, z);
-    float g100 = grad3(hash3(x1, y0, z0, s), x - 1.0f, y, z);
-    float g010 = grad3(hash3(x0, y1, z0, s), x, y - 1.0f, z);
-    float g110 = grad3(hash3(x1, y1, z0, s), x - 1.0f, y - 1.0f, z);
-    float g001 = grad3(hash3(x0, y0, z1, s), x, y, z - 1.0f);
-    float g101 = grad3(hash3(x1, y0, z1, s), x - 1.0f, y, z - 1.0f);
-    float g011 = grad3(hash3(x0, y1, z1, s), x, y - 1.0f, z - 1.0f);
-    float g111 = grad3(hash3(x1, y1, z1, s), x - 1.0f, y - 1.0f, z - 1.0f);
-    float a00 = lerpf(g000, g100, u), a10 = lerpf(g010, g110, u);
-    float a01 = lerpf(g001, g101, u), a11 = lerpf(g011, g111, u);
-    float b0 = lerpf(a00, a10, v), b1 = lerpf(a01, a11, v);
-    return lerpf(b0, b1, w);
-}
-
-__device__ float perlin_fbm3(float x, float y, float z, int F, int octaves, uint32_t s) {
-    float sum = 0.0f, amp = 1.0f, tot = 0.0f;
-    int f = F;
-    for (int o = 0; o < octaves; ++o) {
-        float ff = (float)f;
-        sum = sum + amp * perlin3(x * ff, y * ff, z * ff, f, s + (uint32_t)o);
-        tot = tot + amp;
-        amp = amp * 0.5f;
-        f *= 2;
-    }
-    return sum / tot;
-}
-
 __device__ __forceinline__ float grad2(uint32_t h, float x, float y) {
     switch (h & 7u) {
         case 0: return x + y;
@@ -167,43 +117,241 @@ __device__ float perlin_fbm2(float x, float y, int F, int octaves, uint32_t s) {
 
 __device__ __forceinline__ uint32_t q8(float v) { return (uint32_t)(int)floorf(clamp01(v) * 255.0f + 0.5f); }
 
-__device__ __forceinline__ void put(const NoiseOut& o, size_t i, float r, float g, float b, float a) {
+// A texel in its three storages; channels clamped to [0, 1].
+struct Texel {
+    uint32_t u8;
+    uint2 h16, b16;
+};
+__device__ __forceinline__ Texel make_texel(float r, float g, float b, float a) {
     r = clamp01(r);
     g = clamp01(g);
     b = clamp01(b);
     a = clamp01(a);
-    if (o.u8) o.u8[i] = q8(r) | (q8(g) << 8) | (q8(b) << 16) | (q8(a) << 24);
-    if (o.h16) {
-        uint32_t lo = (uint32_t)__half_as_ushort(__float2half_rn(r)) |
-                      ((uint32_t)__half_as_ushort(__float2half_rn(g)) << 16);
-        uint32_t hi = (uint32_t)__half_as_ushort(__float2half_rn(b)) |
-                      ((uint32_t)__half_as_ushort(__float2half_rn(a)) << 16);
-        o.h16[i] = make_uint2(lo, hi);
-    }
-    if (o.b16) {
-        uint32_t lo = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(r)) |
-                      ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(g)) << 16);
-        uint32_t hi = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(b)) |
-                      ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(a)) << 16);
-        o.b16[i] = make_uint2(lo, hi);
+    Texel t;
+    t.u8 = q8(r) | (q8(g) << 8) | (q8(b) << 16) | (q8(a) << 24);
+    const __half2 hl = __floats2half2_rn(r, g), hh = __floats2half2_rn(b, a);
+    t.h16 = make_uint2(*reinterpret_cast<const uint32_t*>(&hl), *reinterpret_cast<const uint32_t*>(&hh));
+    const __nv_bfloat162 bl = __floats2bfloat162_rn(r, g), bh = __floats2bfloat162_rn(b, a);
+    t.b16 = make_uint2(*reinterpret_cast<const uint32_t*>(&bl), *reinterpret_cast<const uint32_t*>(&bh));
+    return t;
+}
+__device__ __forceinline__ void put(const NoiseOut& o, size_t i, float r, float g, float b, float a) {
+    const Texel t = make_texel(r, g, b, a);
+    o.u8[i] = t.u8;
+    o.h16[i] = t.h16;
+    o.b16[i] = t.b16;
+}
+
+// ---------------------------------------------------------------------------
+// 128^3: R Perlin-Worley, G/B/A Worley fBm at base frequencies 4/8/16 (octaves
+// F, 2F, 4F).  ALU-bound: every texel looks at 27 feature points in each of
+// nine Worley octaves and at 8 corners in each of four Perlin octaves.
+//
+// A thread owns the 2x2x2 texels at even coordinates: in every octave (at most
+// 64 cells over 128 texels) they lie in one cell, so they share each feature
+// point's unpacking, its three pairs of offsets and squares, and the Perlin
+// corners' gradients.  A block owns 32x8x8 texels and hashes the feature points
+// of its cells and their neighbours once, into shared memory (1229 words).
+//
+// The Worley part is exact whatever the order of its operations: in units of
+// 1/1024 cell a feature point is a whole number below 1024 and so is a texel
+// centre's position in its cell ((2x + 1) F / 256 cells, F at least 4), so
+// offsets are whole numbers below 2048 and a squared distance is one below
+// 2^24.  Offsets come from the hash's 10-bit fields dropped into the mantissa
+// of a power of two.  The Perlin part's corner dot products are sums of
+// multiples of 1/256 below 4, exact too; its fades and lerps keep their order.
+//
+// One thread per texel, hashing as it went, the kernel took 766 us (ncu, cold
+// caches); now 131 us.
+// ---------------------------------------------------------------------------
+constexpr int kTileX = 32, kTileY = 8, kTileZ = 8;
+
+// The cells of frequency F a tile touches, with a neighbour on either side.
+template <int F> struct TileCells {
+    static constexpr int along(int texels) { return (texels * F / MT_BASE_N > 1 ? texels * F / MT_BASE_N : 1) + 2; }
+    static constexpr int NX = along(kTileX), NY = along(kTileY), NZ = along(kTileZ), COUNT = NX * NY * NZ;
+};
+
+template <int F> __device__ __forceinline__ void hash_cells(uint32_t* cells, int x0, int y0, int z0, uint32_t s) {
+    using T = TileCells<F>;
+    const int cx = x0 * F / MT_BASE_N - 1, cy = y0 * F / MT_BASE_N - 1, cz = z0 * F / MT_BASE_N - 1;
+    for (int i = threadIdx.x; i < T::COUNT; i += blockDim.x) {
+        const int ix = i % T::NX, iy = (i / T::NX) % T::NY, iz = i / (T::NX * T::NY);
+        cells[i] = hash3((uint32_t)(cx + ix) & (F - 1u), (uint32_t)(cy + iy) & (F - 1u),
+                         (uint32_t)(cz + iz) & (F - 1u), s);
     }
 }
 
-// 128^3: R Perlin-Worley, G/B/A Worley fBm at base frequencies 4/8/16.
-__global__ void __launch_bounds__(128) gen_base_kernel(uint32_t s, NoiseOut o) {
-    const int N = MT_BASE_N;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (uint32_t)(N * N * N)) return;
-    const int x = (int)(i % N), y = (int)((i / N) % N), z = (int)(i / (N * N));
-    const float inv = 1.0f / (float)N;
-    float px = ((float)x + 0.5f) * inv, py = ((float)y + 0.5f) * inv, pz = ((float)z + 0.5f) * inv;
-    float pf = perlin_fbm3(px, py, pz, 4, 4, salt(s, 1));
-    float p01 = clamp01(pf * 0.5f + 0.5f);
-    float g = worley_fbm3(px, py, pz, 4, salt(s, 2));
-    float b = worley_fbm3(px, py, pz, 8, salt(s, 3));
-    float a = worley_fbm3(px, py, pz, 16, salt(s, 4));
-    float r = (p01 - (g - 1.0f)) / (1.0f - (g - 1.0f));
-    put(o, i, r, g, b, a);
+// Inverted Worley noise at frequency F of the texels (x, y, z) + {0, 1}^3 (x
+// fastest); (x, y, z) even, inside the tile at (x0, y0, z0).
+template <int F>
+__device__ __forceinline__ void worley8(float w[8], const uint32_t* cells, int x0, int y0, int z0, int x, int y,
+                                        int z) {
+    using T = TileCells<F>;
+    const int cx = x * F / MT_BASE_N - x0 * F / MT_BASE_N, cy = y * F / MT_BASE_N - y0 * F / MT_BASE_N,
+              cz = z * F / MT_BASE_N - z0 * F / MT_BASE_N;
+    const uint32_t* base = cells + (cz * T::NY + cy) * T::NX + cx;
+    // a texel centre's offset in its cell, in 1/1024 cell; the next texel's is 8F on
+    const float rx = (float)(((2 * x + 1) * F * 4) & 1023), ry = (float)(((2 * y + 1) * F * 4) & 1023),
+                rz = (float)(((2 * z + 1) * F * 4) & 1023);
+    // squared distances as their bits (non-negative floats order like integers),
+    // for the three-input integer minimum
+    int best[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) best[i] = __float_as_int(100.0f * 1048576.0f);
+#pragma unroll 1
+    for (int dz = 0; dz < 3; ++dz) {
+        const float bz = 8192.0f + (rz - (float)(1024 * (dz - 1)));
+#pragma unroll 1
+        for (int dy = 0; dy < 3; ++dy) {
+            const float by = 8192.0f + (ry - (float)(1024 * (dy - 1)));
+            const uint32_t* row = base + (dz * T::NY + dy) * T::NX;
+            int d2[3][8];
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+                const uint32_t h = row[dx];
+                const float bx = 8388608.0f + (rx - (float)(1024 * (dx - 1)));
+                // 2^23 + the field at bit 0, 2^13 + the field at bit 10
+                const float X = __uint_as_float((h & 1023u) | 0x4B000000u) - bx;
+                const float Y = __uint_as_float((h & 0xFFC00u) | 0x46000000u) - by;
+                const float Z = __uint_as_float(((h >> 10) & 0xFFC00u) | 0x46000000u) - bz;
+                const float X1 = X - 8.0f * F, Y1 = Y - 8.0f * F, Z1 = Z - 8.0f * F;
+                const float xx[2] = {X * X, X1 * X1};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float yv = (i & 2) ? Y1 : Y, xy = fmaf(yv, yv, xx[i & 1]);
+                    d2[dx][i] = __float_as_int(fmaf(Z, Z, xy));
+                    d2[dx][i + 4] = __float_as_int(fmaf(Z1, Z1, xy));
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) best[i] = min(__vimin3_s32(best[i], d2[0][i], d2[1][i]), d2[2][i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float d = sqrtf(__int_as_float(best[i]) * (1.0f / 1048576.0f));
+        w[i] = 1.0f - (d < 1.0f ? d : 1.0f);
+    }
+}
+
+// The three octaves F, 2F, 4F over the cells at c, summed into out as they come.
+template <int F>
+__device__ __forceinline__ void worley_fbm8(float out[8], const uint32_t* c, int x0, int y0, int z0, int x, int y,
+                                            int z) {
+    float w[8];
+    worley8<F>(w, c, x0, y0, z0, x, y, z);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) out[i] = w[i] * 0.625f;
+    c += TileCells<F>::COUNT;
+    worley8<2 * F>(w, c, x0, y0, z0, x, y, z);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) out[i] = out[i] + w[i] * 0.25f;
+    c += TileCells<2 * F>::COUNT;
+    worley8<4 * F>(w, c, x0, y0, z0, x, y, z);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) out[i] = out[i] + w[i] * 0.125f;
+}
+template <int F> __device__ __forceinline__ void hash_fbm(uint32_t* c, int x0, int y0, int z0, uint32_t s) {
+    hash_cells<F>(c, x0, y0, z0, s);
+    hash_cells<2 * F>(c + TileCells<F>::COUNT, x0, y0, z0, s + 1u);
+    hash_cells<4 * F>(c + TileCells<F>::COUNT + TileCells<2 * F>::COUNT, x0, y0, z0, s + 2u);
+}
+template <int F> constexpr int kFbmCells = TileCells<F>::COUNT + TileCells<2 * F>::COUNT + TileCells<4 * F>::COUNT;
+
+// Perlin's gradient of a corner's hash as a vector of -1, 0, 1: the dot product
+// is one of x, y plus or minus one of y, x, z.
+__device__ __forceinline__ void grad3(uint32_t h, float& gx, float& gy, float& gz) {
+    h &= 15u;
+    const float su = (h & 1u) ? -1.0f : 1.0f, sv = (h & 2u) ? -1.0f : 1.0f;
+    const bool u_is_x = h < 8u, v_is_y = h < 4u, v_is_x = h == 12u || h == 14u;
+    gx = u_is_x ? su : (v_is_x ? sv : 0.0f);
+    gy = u_is_x ? (v_is_y ? sv : 0.0f) : su;
+    gz = (v_is_y || v_is_x) ? 0.0f : sv;
+}
+
+// Perlin noise at frequency F of the eight texels.
+__device__ __forceinline__ void perlin8(float out[8], int x, int y, int z, int F, uint32_t s) {
+    const uint32_t m = (uint32_t)F - 1u;
+    const uint32_t cx = (uint32_t)(x * F / MT_BASE_N), cy = (uint32_t)(y * F / MT_BASE_N),
+                   cz = (uint32_t)(z * F / MT_BASE_N);
+    float px[2], py[2], pz[2], u[2], v[2], w[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        px[i] = (float)(((2 * (x + i) + 1) * F) & 255) * (1.0f / 256.0f);
+        py[i] = (float)(((2 * (y + i) + 1) * F) & 255) * (1.0f / 256.0f);
+        pz[i] = (float)(((2 * (z + i) + 1) * F) & 255) * (1.0f / 256.0f);
+        u[i] = fade(px[i]);
+        v[i] = fade(py[i]);
+        w[i] = fade(pz[i]);
+    }
+    float plane[2][8];  // the bilinear blend of each z plane's corners, per texel
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        float a[2][8];  // the blend along x of each row's corners
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            float g[2][8];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                float gx, gy, gz;
+                grad3(hash3((cx + (uint32_t)k) & m, (cy + (uint32_t)b) & m, (cz + (uint32_t)c) & m, s), gx, gy, gz);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    g[k][i] = gx * (px[i & 1] - (float)k) + gy * (py[(i >> 1) & 1] - (float)b) +
+                              gz * (pz[i >> 2] - (float)c);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[b][i] = lerpf(g[0][i], g[1][i], u[i & 1]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) plane[c][i] = lerpf(a[0][i], a[1][i], v[(i >> 1) & 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) out[i] = lerpf(plane[0][i], plane[1][i], w[i >> 2]);
+}
+
+__global__ void __launch_bounds__(256, 3) gen_base_kernel(uint32_t s, NoiseOut o) {
+    constexpr int N = MT_BASE_N;
+    __shared__ uint32_t cells[kFbmCells<4> + kFbmCells<8> + kFbmCells<16>];
+    const int x0 = (int)blockIdx.x * kTileX, y0 = (int)blockIdx.y * kTileY, z0 = (int)blockIdx.z * kTileZ;
+    hash_fbm<4>(cells, x0, y0, z0, salt(s, 2));
+    hash_fbm<8>(cells + kFbmCells<4>, x0, y0, z0, salt(s, 3));
+    hash_fbm<16>(cells + kFbmCells<4> + kFbmCells<8>, x0, y0, z0, salt(s, 4));
+    __syncthreads();
+    const int tid = (int)threadIdx.x;
+    const int x = x0 + 2 * (tid & 15), y = y0 + 2 * ((tid >> 4) & 3), z = z0 + 2 * (tid >> 6);
+    float r[8], g[8], b[8], a[8];
+    {
+        // perlin_fbm: octaves 4, 8, 16, 32 at amplitudes 1, 1/2, 1/4, 1/8
+        float amp = 1.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = 0.0f;
+#pragma unroll 1
+        for (int oct = 0; oct < 4; ++oct) {
+            float p[8];
+            perlin8(p, x, y, z, 4 << oct, salt(s, 1) + (uint32_t)oct);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) r[i] = r[i] + amp * p[i];
+            amp = amp * 0.5f;
+        }
+    }
+    worley_fbm8<4>(g, cells, x0, y0, z0, x, y, z);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float p01 = clamp01((r[i] / 1.875f) * 0.5f + 0.5f);
+        r[i] = (p01 - (g[i] - 1.0f)) / (1.0f - (g[i] - 1.0f));
+    }
+    worley_fbm8<8>(b, cells + kFbmCells<4>, x0, y0, z0, x, y, z);
+    worley_fbm8<16>(a, cells + kFbmCells<4> + kFbmCells<8>, x0, y0, z0, x, y, z);
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {  // the two texels of a row as one store per storage
+        const size_t at = (((size_t)(z + (i >> 2)) * N + (size_t)(y + ((i >> 1) & 1))) * N + (size_t)x) / 2;
+        const Texel t0 = make_texel(r[i], g[i], b[i], a[i]), t1 = make_texel(r[i + 1], g[i + 1], b[i + 1], a[i + 1]);
+        reinterpret_cast<uint2*>(o.u8)[at] = make_uint2(t0.u8, t1.u8);
+        reinterpret_cast<uint4*>(o.h16)[at] = make_uint4(t0.h16.x, t0.h16.y, t1.h16.x, t1.h16.y);
+        reinterpret_cast<uint4*>(o.b16)[at] = make_uint4(t0.b16.x, t0.b16.y, t1.b16.x, t1.b16.y);
+    }
 }
 
 // 32^3: Worley at frequencies 8/16/32 in R/G/B.
@@ -258,9 +406,10 @@ __global__ void u8_to_16_kernel(const uint32_t* __restrict__ src, size_t n, uint
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t v = src[i];
-    NoiseOut o{nullptr, h16, b16};
-    put(o, i, (float)(v & 0xffu) / 255.0f, (float)((v >> 8) & 0xffu) / 255.0f, (float)((v >> 16) & 0xffu) / 255.0f,
-        (float)(v >> 24) / 255.0f);
+    const Texel t = make_texel((float)(v & 0xffu) / 255.0f, (float)((v >> 8) & 0xffu) / 255.0f,
+                               (float)((v >> 16) & 0xffu) / 255.0f, (float)(v >> 24) / 255.0f);
+    h16[i] = t.h16;
+    b16[i] = t.b16;
 }
 
 // Plane-quad layout of an RGBA8 volume (what the plain form's 3D samplers
@@ -327,8 +476,8 @@ cudaError_t launch_cells2(const uint32_t* img, int n, uint4* cells, cudaStream_t
 }
 
 cudaError_t launch_generate_base(uint32_t seed, NoiseOut o, cudaStream_t s) {
-    const unsigned n = MT_BASE_N * MT_BASE_N * MT_BASE_N;
-    gen_base_kernel<<<(n + 127) / 128, 128, 0, s>>>(seed, o);
+    const dim3 grid(MT_BASE_N / kTileX, MT_BASE_N / kTileY, MT_BASE_N / kTileZ);
+    gen_base_kernel<<<grid, 256, 0, s>>>(seed, o);
     return cudaGetLastError();
 }
 cudaError_t launch_generate_detail(uint32_t seed, NoiseOut o, cudaStream_t s) {
