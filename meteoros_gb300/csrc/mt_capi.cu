@@ -158,16 +158,20 @@ mt_status ensure_weather(mt_ctx* ctx, int slot) {
     return alloc(ctx, &ctx->weather16[1][slot], kWeatherTexels);
 }
 
-// The plane-quad copies of a volume's two 16-bit versions, after they change.
-cudaError_t refresh_quads(mt_ctx* ctx, int volume, cudaStream_t s) {
-    const bool base = volume == MT_VOLUME_BASE;
-    for (int k = 0; k < 2; ++k) {
-        const cudaError_t e = mt::launch_quads16(base ? ctx->base16[k] : ctx->detail16[k],
-                                                 base ? MT_BASE_N : MT_DETAIL_N,
-                                                 base ? ctx->base16q[k] : ctx->detail16q[k], s);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+// What launch_layouts makes of each volume when it changes.
+mt::LayoutJob base_job(mt_ctx* c) {
+    return mt::LayoutJob{c->base, c->base16[0], c->base16[1], c->base_c, c->base16q[0], c->base16q[1], MT_BASE_N};
+}
+mt::LayoutJob detail_job(mt_ctx* c) {
+    return mt::LayoutJob{c->detail, c->detail16[0], c->detail16[1], c->detail_c, c->detail16q[0], c->detail16q[1],
+                         MT_DETAIL_N};
+}
+mt::LayoutJob curl_job(mt_ctx* c) {
+    return mt::LayoutJob{c->curl, c->curl16[0], c->curl16[1], c->curl_c, nullptr, nullptr, MT_CURL_N};
+}
+mt::LayoutJob weather_job(mt_ctx* c, int slot) {
+    return mt::LayoutJob{c->weather[slot], c->weather16[0][slot], c->weather16[1][slot], c->weather_c[slot], nullptr,
+                         nullptr, MT_WEATHER_N};
 }
 
 mt_status ensure_volumes(mt_ctx* ctx) {
@@ -340,29 +344,29 @@ MT_API mt_status mt_upload_volumes(mt_ctx* ctx, const uint8_t* base, const uint8
     mt_status st;
     if ((st = bind_device(ctx)) != MT_OK) return st;
     if ((st = ensure_volumes(ctx)) != MT_OK) return st;
+    if (weather && (st = ensure_weather(ctx, 0)) != MT_OK) return st;
+    mt::LayoutJob jobs[mt::kMaxLayoutJobs];
+    int n = 0;
     if (base) {
         MT_CUDA(ctx, cudaMemcpy(ctx->base, base, kBaseTexels * 4, cudaMemcpyHostToDevice));
-        MT_CUDA(ctx, mt::launch_u8_to_16(ctx->base, kBaseTexels, ctx->base16[0], ctx->base16[1], 0));
-        MT_CUDA(ctx, mt::launch_quads3(ctx->base, MT_BASE_N, ctx->base_c, 0));
-        MT_CUDA(ctx, refresh_quads(ctx, MT_VOLUME_BASE, 0));
-        ctx->have_base = true;
+        jobs[n++] = base_job(ctx);
     }
     if (detail) {
         MT_CUDA(ctx, cudaMemcpy(ctx->detail, detail, kDetailTexels * 4, cudaMemcpyHostToDevice));
-        MT_CUDA(ctx, mt::launch_u8_to_16(ctx->detail, kDetailTexels, ctx->detail16[0], ctx->detail16[1], 0));
-        MT_CUDA(ctx, mt::launch_quads3(ctx->detail, MT_DETAIL_N, ctx->detail_c, 0));
-        MT_CUDA(ctx, refresh_quads(ctx, MT_VOLUME_DETAIL, 0));
-        ctx->have_detail = true;
+        jobs[n++] = detail_job(ctx);
     }
     if (curl) {
         MT_CUDA(ctx, cudaMemcpy(ctx->curl, curl, kCurlTexels * 4, cudaMemcpyHostToDevice));
-        MT_CUDA(ctx, mt::launch_u8_to_16(ctx->curl, kCurlTexels, ctx->curl16[0], ctx->curl16[1], 0));
-        MT_CUDA(ctx, mt::launch_cells2(ctx->curl, MT_CURL_N, ctx->curl_c, 0));
-        ctx->have_curl = true;
+        jobs[n++] = curl_job(ctx);
     }
     if (weather) {
-        if ((st = mt_upload_weather(ctx, 0, weather)) != MT_OK) return st;
+        MT_CUDA(ctx, cudaMemcpy(ctx->weather[0], weather, kWeatherTexels * 4, cudaMemcpyHostToDevice));
+        jobs[n++] = weather_job(ctx, 0);
     }
+    MT_CUDA(ctx, mt::launch_layouts(jobs, n, true, 0));
+    ctx->have_base = ctx->have_base || base;
+    ctx->have_detail = ctx->have_detail || detail;
+    ctx->have_curl = ctx->have_curl || curl;
     MT_CUDA(ctx, cudaDeviceSynchronize());
     return MT_OK;
 }
@@ -410,12 +414,8 @@ MT_API mt_status mt_decode_tga_volume(mt_ctx* ctx, int volume, const uint8_t* co
     if (e == cudaSuccess)
         e = cudaMemcpy(d_table, table.data(), table.size() * sizeof(mt::TgaSlice), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = mt::launch_tga_decode(d_blob, d_table, n, max_size, vol, n, n, s);
-    const size_t texels = (size_t)n * n * n;
-    if (e == cudaSuccess)
-        e = mt::launch_u8_to_16(vol, texels, volume == MT_VOLUME_BASE ? ctx->base16[0] : ctx->detail16[0],
-                                volume == MT_VOLUME_BASE ? ctx->base16[1] : ctx->detail16[1], s);
-    if (e == cudaSuccess) e = mt::launch_quads3(vol, n, volume == MT_VOLUME_BASE ? ctx->base_c : ctx->detail_c, s);
-    if (e == cudaSuccess) e = refresh_quads(ctx, volume, s);
+    const mt::LayoutJob job = volume == MT_VOLUME_BASE ? base_job(ctx) : detail_job(ctx);
+    if (e == cudaSuccess) e = mt::launch_layouts(&job, 1, true, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cudaFree(d_blob);
     cudaFree(d_table);
@@ -437,9 +437,8 @@ MT_API mt_status mt_upload_weather(mt_ctx* ctx, int slot, const uint8_t* weather
     if ((st = bind_device(ctx)) != MT_OK) return st;
     if ((st = ensure_weather(ctx, slot)) != MT_OK) return st;
     MT_CUDA(ctx, cudaMemcpy(ctx->weather[slot], weather, kWeatherTexels * 4, cudaMemcpyHostToDevice));
-    MT_CUDA(ctx, mt::launch_u8_to_16(ctx->weather[slot], kWeatherTexels, ctx->weather16[0][slot],
-                                     ctx->weather16[1][slot], 0));
-    MT_CUDA(ctx, mt::launch_cells2(ctx->weather[slot], MT_WEATHER_N, ctx->weather_c[slot], 0));
+    const mt::LayoutJob job = weather_job(ctx, slot);
+    MT_CUDA(ctx, mt::launch_layouts(&job, 1, true, 0));
     MT_CUDA(ctx, cudaDeviceSynchronize());
     return MT_OK;
 }
@@ -449,18 +448,15 @@ MT_API mt_status mt_generate_volumes(mt_ctx* ctx, uint64_t seed, void* stream) {
     mt_status st;
     if ((st = bind_device(ctx)) != MT_OK) return st;
     if ((st = ensure_volumes(ctx)) != MT_OK) return st;
+    if ((st = ensure_weather(ctx, 0)) != MT_OK) return st;
     cudaStream_t s = (cudaStream_t)stream;
-    const uint32_t s32 = seed32(seed);
-    MT_CUDA(ctx, mt::launch_generate_base(s32, mt::NoiseOut{ctx->base, ctx->base16[0], ctx->base16[1]}, s));
-    MT_CUDA(ctx, mt::launch_generate_detail(s32, mt::NoiseOut{ctx->detail, ctx->detail16[0], ctx->detail16[1]}, s));
-    MT_CUDA(ctx, mt::launch_generate_curl(s32, mt::NoiseOut{ctx->curl, ctx->curl16[0], ctx->curl16[1]}, s));
-    MT_CUDA(ctx, mt::launch_quads3(ctx->base, MT_BASE_N, ctx->base_c, s));
-    MT_CUDA(ctx, mt::launch_quads3(ctx->detail, MT_DETAIL_N, ctx->detail_c, s));
-    MT_CUDA(ctx, mt::launch_cells2(ctx->curl, MT_CURL_N, ctx->curl_c, s));
-    MT_CUDA(ctx, refresh_quads(ctx, MT_VOLUME_BASE, s));
-    MT_CUDA(ctx, refresh_quads(ctx, MT_VOLUME_DETAIL, s));
+    const mt::LayoutJob jobs[4] = {base_job(ctx), detail_job(ctx), curl_job(ctx), weather_job(ctx, 0)};
+    mt::NoiseOut out[4];
+    for (int k = 0; k < 4; ++k) out[k] = mt::NoiseOut{const_cast<uint32_t*>(jobs[k].u8), jobs[k].h16, jobs[k].b16};
+    MT_CUDA(ctx, mt::launch_generate_volumes(seed32(seed), out[0], out[1], out[2], out[3], s));
+    MT_CUDA(ctx, mt::launch_layouts(jobs, 4, false, s));
     ctx->have_base = ctx->have_detail = ctx->have_curl = true;
-    return mt_generate_weather(ctx, 0, seed, stream);
+    return MT_OK;
 }
 
 MT_API mt_status mt_generate_weather(mt_ctx* ctx, int slot, uint64_t seed, void* stream) {
@@ -472,7 +468,8 @@ MT_API mt_status mt_generate_weather(mt_ctx* ctx, int slot, uint64_t seed, void*
     MT_CUDA(ctx, mt::launch_generate_weather(
                      seed32(seed), mt::NoiseOut{ctx->weather[slot], ctx->weather16[0][slot], ctx->weather16[1][slot]},
                      (cudaStream_t)stream));
-    MT_CUDA(ctx, mt::launch_cells2(ctx->weather[slot], MT_WEATHER_N, ctx->weather_c[slot], (cudaStream_t)stream));
+    const mt::LayoutJob job = weather_job(ctx, slot);
+    MT_CUDA(ctx, mt::launch_layouts(&job, 1, false, (cudaStream_t)stream));
     return MT_OK;
 }
 

@@ -74,9 +74,9 @@ struct MarchArgs {
     mt_params params;
     // base (MT_BASE_N^3), detail (MT_DETAIL_N^3), curl (MT_CURL_N^2), weather
     // (MT_WEATHER_N^2, slot params.weather_slot) in params.storage: for RGBA8
-    // plane quads of the volumes and bilinear cells of the images (uint4;
-    // launch_quads3 / launch_cells2), for the 16-bit storages plane quads of
-    // the volumes (2 x uint4; launch_quads16) and four 16-bit values per texel
+    // plane quads of the volumes and bilinear cells of the images (uint4), for
+    // the 16-bit storages plane quads of the volumes (2 x uint4), all as
+    // launch_layouts makes them, and four 16-bit values per texel
     // (uint2) of the images
     const void* vol[4];
     const float4* prev;
@@ -237,18 +237,22 @@ cudaError_t launch_tonemap(const TonemapArgs& a, cudaStream_t s);
 cudaError_t launch_frame(const MarchArgs& a, cudaStream_t s, const LaunchEvents* ev, const ForkJoin* fj);
 cudaError_t launch_selftest_division(const float* a, const float* b, float* out_rdiv, float* out_ieee, int n,
                                      cudaStream_t s);
-cudaError_t launch_generate_base(uint32_t seed, NoiseOut o, cudaStream_t s);
-cudaError_t launch_generate_detail(uint32_t seed, NoiseOut o, cudaStream_t s);
-cudaError_t launch_generate_curl(uint32_t seed, NoiseOut o, cudaStream_t s);
+cudaError_t launch_generate_volumes(uint32_t seed, NoiseOut base, NoiseOut detail, NoiseOut curl, NoiseOut weather,
+                                    cudaStream_t s);
 cudaError_t launch_generate_weather(uint32_t seed, NoiseOut o, cudaStream_t s);
-cudaError_t launch_u8_to_16(const uint32_t* src, size_t n, uint2* h16, uint2* b16, cudaStream_t s);
-// The layouts the plain form's samplers read: plane quads of an RGBA8 volume
-// (n^3 x uint4) and bilinear cells of an RGBA8 image (n^2 x uint4).
-cudaError_t launch_quads3(const uint32_t* vol, int n, uint4* quads, cudaStream_t s);
-cudaError_t launch_cells2(const uint32_t* img, int n, uint4* cells, cudaStream_t s);
-// Plane-quad copies of a 16-bit volume (n^3 entries of 2 x uint4), the layout
-// the precision form's 3D samplers read.
-cudaError_t launch_quads16(const uint2* vol, int n, uint4* quads, cudaStream_t s);
+// The layouts the samplers read, of up to kMaxLayoutJobs volumes and images in
+// one launch (mt_noise.cu); from_u8: their 16-bit texels too.
+constexpr int kMaxLayoutJobs = 4;
+struct LayoutJob {
+    const uint32_t* u8;  // the texels in their three storages
+    uint2* h16;
+    uint2* b16;
+    uint4* quads;        // RGBA8: n^3 plane quads, or n^2 bilinear cells of an image
+    uint4* quads_h16;    // 16-bit plane quads (n^3 x 2); NULL: an image, which has none
+    uint4* quads_b16;
+    int32_t n;           // texels on an axis
+};
+cudaError_t launch_layouts(const LayoutJob* jobs, int n_jobs, bool from_u8, cudaStream_t s);
 
 // Number of 4x4 blocks along one axis covered by the reference's raymarch
 // dispatch: ceil(floor(dim/4) / 32) groups of 32 (Renderer.cpp:713-716).

@@ -20,8 +20,8 @@ template <int S> struct Vol;
 // T3: the element of the 3D volumes (base, detail), T2: of the 2D images
 // (curl, weather), as build_march_args points at them.
 template <> struct Vol<MT_STORAGE_U8> {
-    using T3 = uint4;  // plane quads (launch_quads3)
-    using T2 = uint4;  // bilinear cells (launch_cells2)
+    using T3 = uint4;  // plane quads (launch_layouts)
+    using T2 = uint4;  // bilinear cells (launch_layouts)
     template <int N> static MT_HD f4v tex3(const T3* v, f3 s) { return tex3_u8<N>(v, s); }
     template <int N> static MT_HD f4v tex3_light(const T3* v, f3 s) { return tex3_u8_fused<N>(v, s); }
     template <int N> static MT_HD f4v tex2(const T2* v, float x, float y) { return tex2_u8<N>(v, x, y); }
@@ -31,7 +31,7 @@ template <> struct Vol<MT_STORAGE_U8> {
 // in-cloud step, which reach colour only and run in half2 (lerps and density
 // math, sample_light_pair).
 template <class P> struct Vol16 {
-    using T3 = uint4;  // plane quads (launch_quads16)
+    using T3 = uint4;  // plane quads (launch_layouts)
     using T2 = uint2;
     template <int N> static MT_HD f4v tex3(const T3* v, f3 s) { return tex3_p16q_f32<N, P>(v, s); }
     // bfloat16 (an 8-bit mantissa) filters its cone-light samples in FP32 too

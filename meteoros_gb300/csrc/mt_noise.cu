@@ -162,7 +162,8 @@ __device__ __forceinline__ void put(const NoiseOut& o, size_t i, float r, float 
 // multiples of 1/256 below 4, exact too; its fades and lerps keep their order.
 //
 // One thread per texel, hashing as it went, the kernel took 766 us (ncu, cold
-// caches); now 131 us.
+// caches); now 131 us with the small outputs beside it.  All of mt_generate_volumes:
+// 864 -> 164 us.
 // ---------------------------------------------------------------------------
 constexpr int kTileX = 32, kTileY = 8, kTileZ = 8;
 
@@ -311,10 +312,10 @@ __device__ __forceinline__ void perlin8(float out[8], int x, int y, int z, int F
     for (int i = 0; i < 8; ++i) out[i] = lerpf(plane[0][i], plane[1][i], w[i >> 2]);
 }
 
-__global__ void __launch_bounds__(256, 3) gen_base_kernel(uint32_t s, NoiseOut o) {
-    constexpr int N = MT_BASE_N;
+__device__ __forceinline__ void gen_base_tile(uint32_t s, const NoiseOut& o, int tile) {
+    constexpr int N = MT_BASE_N, TX = N / kTileX, TY = N / kTileY;
     __shared__ uint32_t cells[kFbmCells<4> + kFbmCells<8> + kFbmCells<16>];
-    const int x0 = (int)blockIdx.x * kTileX, y0 = (int)blockIdx.y * kTileY, z0 = (int)blockIdx.z * kTileZ;
+    const int x0 = tile % TX * kTileX, y0 = tile / TX % TY * kTileY, z0 = tile / (TX * TY) * kTileZ;
     hash_fbm<4>(cells, x0, y0, z0, salt(s, 2));
     hash_fbm<8>(cells + kFbmCells<4>, x0, y0, z0, salt(s, 3));
     hash_fbm<16>(cells + kFbmCells<4> + kFbmCells<8>, x0, y0, z0, salt(s, 4));
@@ -355,10 +356,8 @@ __global__ void __launch_bounds__(256, 3) gen_base_kernel(uint32_t s, NoiseOut o
 }
 
 // 32^3: Worley at frequencies 8/16/32 in R/G/B.
-__global__ void __launch_bounds__(128) gen_detail_kernel(uint32_t s, NoiseOut o) {
+__device__ __forceinline__ void gen_detail_texel(uint32_t s, const NoiseOut& o, uint32_t i) {
     const int N = MT_DETAIL_N;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (uint32_t)(N * N * N)) return;
     const int x = (int)(i % N), y = (int)((i / N) % N), z = (int)(i / (N * N));
     const float inv = 1.0f / (float)N;
     float px = ((float)x + 0.5f) * inv, py = ((float)y + 0.5f) * inv, pz = ((float)z + 0.5f) * inv;
@@ -369,10 +368,8 @@ __global__ void __launch_bounds__(128) gen_detail_kernel(uint32_t s, NoiseOut o)
 }
 
 // 128^2 curl of a tileable Perlin fBm potential (central differences).
-__global__ void __launch_bounds__(128) gen_curl_kernel(uint32_t s, NoiseOut o) {
+__device__ __forceinline__ void gen_curl_texel(uint32_t s, const NoiseOut& o, uint32_t i) {
     const int N = MT_CURL_N;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (uint32_t)(N * N)) return;
     const int x = (int)(i % N), y = (int)(i / N);
     const float inv = 1.0f / (float)N;
     float px = ((float)x + 0.5f) * inv, py = ((float)y + 0.5f) * inv;
@@ -386,10 +383,8 @@ __global__ void __launch_bounds__(128) gen_curl_kernel(uint32_t s, NoiseOut o) {
 }
 
 // 512^2 weather: R coverage, G precipitation, B cloud type, A = 1.
-__global__ void __launch_bounds__(128) gen_weather_kernel(uint32_t s, NoiseOut o) {
+__device__ __forceinline__ void gen_weather_texel(uint32_t s, const NoiseOut& o, uint32_t i) {
     const int N = MT_WEATHER_N;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (uint32_t)(N * N)) return;
     const int x = (int)(i % N), y = (int)(i / N);
     const float inv = 1.0f / (float)N;
     float px = ((float)x + 0.5f) * inv, py = ((float)y + 0.5f) * inv;
@@ -401,102 +396,137 @@ __global__ void __launch_bounds__(128) gen_weather_kernel(uint32_t s, NoiseOut o
     put(o, i, cov, precip, type, 1.0f);
 }
 
-// RGBA8 UNORM -> half / bfloat16 copies (c / 255, round to nearest even).
-__global__ void u8_to_16_kernel(const uint32_t* __restrict__ src, size_t n, uint2* h16, uint2* b16) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t v = src[i];
-    const Texel t = make_texel((float)(v & 0xffu) / 255.0f, (float)((v >> 8) & 0xffu) / 255.0f,
-                               (float)((v >> 16) & 0xffu) / 255.0f, (float)(v >> 24) / 255.0f);
-    h16[i] = t.h16;
-    b16[i] = t.b16;
+// One launch for the four outputs: the base volume's tiles first, then the small
+// ones, whose blocks fill its last wave (29 us as three launches of their own).
+constexpr int kGenThreads = 256;
+constexpr int kBaseTiles = (MT_BASE_N / kTileX) * (MT_BASE_N / kTileY) * (MT_BASE_N / kTileZ);
+constexpr int kDetailBlocks = MT_DETAIL_N * MT_DETAIL_N * MT_DETAIL_N / kGenThreads;
+constexpr int kCurlBlocks = MT_CURL_N * MT_CURL_N / kGenThreads;
+constexpr int kWeatherBlocks = MT_WEATHER_N * MT_WEATHER_N / kGenThreads;
+static_assert((kTileX / 2) * (kTileY / 2) * (kTileZ / 2) == kGenThreads, "a thread owns 2x2x2 texels of the tile");
+
+__global__ void __launch_bounds__(kGenThreads, 3) gen_volumes_kernel(uint32_t s, NoiseOut base, NoiseOut detail,
+                                                                     NoiseOut curl, NoiseOut weather) {
+    int block = (int)blockIdx.x;
+    if (block < kBaseTiles) {
+        gen_base_tile(s, base, block);
+        return;
+    }
+    block -= kBaseTiles;
+    if (block < kWeatherBlocks) {
+        gen_weather_texel(s, weather, (uint32_t)(block * kGenThreads) + threadIdx.x);
+        return;
+    }
+    block -= kWeatherBlocks;
+    if (block < kDetailBlocks)
+        gen_detail_texel(s, detail, (uint32_t)(block * kGenThreads) + threadIdx.x);
+    else
+        gen_curl_texel(s, curl, (uint32_t)((block - kDetailBlocks) * kGenThreads) + threadIdx.x);
 }
 
-// Plane-quad layout of an RGBA8 volume (what the plain form's 3D samplers
-// read): entry (x, y, z) holds the four texels of plane z a trilinear fetch
-// at that cell interpolates, {(x0,y0), (x1,y0), (x0,y1), (x1,y1)} with
-// x1 = (x + 1) mod N, y1 likewise (REPEAT), as one 16-byte word: a fetch reads
-// two entries, at z0 and z1.
-__global__ void quads3_kernel(const uint32_t* __restrict__ vol, int n, uint4* __restrict__ quads) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t nn = (size_t)n * n;
-    if (i >= nn * n) return;
-    const unsigned m = (unsigned)n - 1u;
-    const unsigned x = (unsigned)(i % n), y = (unsigned)((i / n) % n), z = (unsigned)(i / nn);
-    const unsigned x1 = (x + 1u) & m, y1 = (y + 1u) & m;
-    const uint32_t* p = vol + (size_t)z * nn;
-    quads[i] = make_uint4(p[y * n + x], p[y * n + x1], p[y1 * n + x], p[y1 * n + x1]);
+__global__ void __launch_bounds__(kGenThreads) gen_weather_kernel(uint32_t s, NoiseOut o) {
+    gen_weather_texel(s, o, blockIdx.x * kGenThreads + threadIdx.x);
 }
 
-// The same for an RGBA8 image (bilinear cells): {(x0,y0), (x1,y0), (x0,y1), (x1,y1)}.
-__global__ void cells2_kernel(const uint32_t* __restrict__ img, int n, uint4* __restrict__ cells) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)n * n) return;
-    const unsigned m = (unsigned)n - 1u;
-    const unsigned x = (unsigned)(i % n), y = (unsigned)(i / n);
-    const unsigned x1 = (x + 1u) & m, y1 = (y + 1u) & m;
-    cells[i] = make_uint4(img[y * n + x], img[y * n + x1], img[y1 * n + x], img[y1 * n + x1]);
+// ---------------------------------------------------------------------------
+// The layouts the samplers read, from a volume's texels, in one pass over every
+// volume that changed (LayoutJob):
+//   * RGBA8 plane quads of a volume, bilinear cells of an image: entry (x, y[,
+//     z]) holds the four texels a fetch at that cell interpolates in plane z,
+//     {(x0,y0), (x1,y0), (x0,y1), (x1,y1)} with x1 = (x + 1) mod N, y1 likewise
+//     (REPEAT), as one 16-byte word;
+//   * the same of a volume's IEEE half and bfloat16 texels, a 32-byte entry
+//     {(x0,y0), (x1,y0)}, {(x0,y1), (x1,y1)} each;
+//   * FROM_U8 (uploaded and decoded volumes): the 16-bit texels themselves,
+//     c / 255 rounded to nearest even.  c * (1 / 255) rounds to the same half and
+//     the same bfloat16 for each of the 256 bytes.
+// Bound by its stores: 96 bytes a texel of the base volume (112 with the 16-bit
+// texels), 32 bytes an instruction.  The four outputs of the generator take
+// 32 us (ncu, cold caches; 201 MB written); one kernel per layout and volume,
+// each reading its input again, took 65, and twelve launches of an upload 98.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void store32(uint4* p, uint2 a, uint2 b, uint2 c, uint2 d) {
+    asm volatile("st.global.v8.u32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(b.x),
+                 "r"(b.y), "r"(c.x), "r"(c.y), "r"(d.x), "r"(d.y)
+                 : "memory");
+}
+__device__ __forceinline__ void u8_to_16(uint32_t v, uint2& h, uint2& b) {
+    const float k = 1.0f / 255.0f;
+    const float c0 = (float)(v & 0xffu) * k, c1 = (float)((v >> 8) & 0xffu) * k, c2 = (float)((v >> 16) & 0xffu) * k,
+                c3 = (float)(v >> 24) * k;
+    const __half2 hl = __floats2half2_rn(c0, c1), hh = __floats2half2_rn(c2, c3);
+    h = make_uint2(*reinterpret_cast<const uint32_t*>(&hl), *reinterpret_cast<const uint32_t*>(&hh));
+    const __nv_bfloat162 bl = __floats2bfloat162_rn(c0, c1), bh = __floats2bfloat162_rn(c2, c3);
+    b = make_uint2(*reinterpret_cast<const uint32_t*>(&bl), *reinterpret_cast<const uint32_t*>(&bh));
 }
 
-// Plane-quad layout of a 16-bit volume (what the precision form's 3D samplers
-// read): entry (x, y, z) holds the four texels of the z plane a trilinear
-// fetch interpolates, as two 16-byte words {(x0,y0), (x1,y0)} and
-// {(x0,y1), (x1,y1)}, x1 = (x + 1) mod N (REPEAT): a fetch reads the entries
-// at z0 and z1, one 32-byte sector each.
-__global__ void quads16_kernel(const uint2* __restrict__ vol, int n, uint4* __restrict__ quads) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t nn = (size_t)n * n;
-    if (i >= nn * n) return;
-    const unsigned m = (unsigned)n - 1u;
-    const unsigned x = (unsigned)(i % n), y = (unsigned)((i / n) % n), z = (unsigned)(i / nn);
-    const unsigned x1 = (x + 1u) & m, y1 = (y + 1u) & m;
-    const uint2* p = vol + (size_t)z * nn;
-    const uint2 a = p[y * n + x], b = p[y * n + x1], c = p[y1 * n + x], d = p[y1 * n + x1];
-    quads[2 * i] = make_uint4(a.x, a.y, b.x, b.y);
-    quads[2 * i + 1] = make_uint4(c.x, c.y, d.x, d.y);
+struct LayoutArgs {
+    LayoutJob job[kMaxLayoutJobs];
+    unsigned first_block[kMaxLayoutJobs + 1];
+    int n_jobs;
+};
+
+template <bool FROM_U8> __global__ void __launch_bounds__(256) layouts_kernel(const __grid_constant__ LayoutArgs a) {
+    int k = 0;
+    while (k + 1 < a.n_jobs && blockIdx.x >= a.first_block[k + 1]) ++k;
+    const LayoutJob& j = a.job[k];
+    const unsigned i = (blockIdx.x - a.first_block[k]) * 256u + threadIdx.x;
+    const unsigned n = (unsigned)j.n, m = n - 1u;
+    const unsigned x = i & m, row = i & ~m, y = (i / n) & m, plane = row - y * n;
+    const unsigned x1 = (x + 1u) & m, row1 = plane + ((y + 1u) & m) * n;
+    const unsigned at[4] = {row + x, row + x1, row1 + x, row1 + x1};
+    uint32_t t[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) t[c] = j.u8[at[c]];
+    j.quads[i] = make_uint4(t[0], t[1], t[2], t[3]);
+    uint2 h[4], b[4];
+    if (FROM_U8) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) u8_to_16(t[c], h[c], b[c]);
+        j.h16[i] = h[0];
+        j.b16[i] = b[0];
+    }
+    if (!j.quads_h16) return;  // an image
+    if (!FROM_U8) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            h[c] = j.h16[at[c]];
+            b[c] = j.b16[at[c]];
+        }
+    }
+    store32(j.quads_h16 + 2u * i, h[0], h[1], h[2], h[3]);
+    store32(j.quads_b16 + 2u * i, b[0], b[1], b[2], b[3]);
 }
 
 }  // namespace
 
-cudaError_t launch_quads16(const uint2* vol, int n, uint4* quads, cudaStream_t s) {
-    const size_t texels = (size_t)n * n * n;
-    quads16_kernel<<<(unsigned)((texels + 255) / 256), 256, 0, s>>>(vol, n, quads);
+cudaError_t launch_layouts(const LayoutJob* jobs, int n_jobs, bool from_u8, cudaStream_t s) {
+    if (n_jobs <= 0) return cudaSuccess;
+    LayoutArgs a = {};
+    a.n_jobs = n_jobs;
+    unsigned blocks = 0;
+    for (int k = 0; k < n_jobs; ++k) {
+        const unsigned n = (unsigned)jobs[k].n;
+        a.job[k] = jobs[k];
+        a.first_block[k] = blocks;
+        blocks += n * n * (jobs[k].quads_h16 ? n : 1u) / 256u;  // n is a power of two, at least 32
+    }
+    a.first_block[n_jobs] = blocks;
+    if (from_u8)
+        layouts_kernel<true><<<blocks, 256, 0, s>>>(a);
+    else
+        layouts_kernel<false><<<blocks, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_quads3(const uint32_t* vol, int n, uint4* quads, cudaStream_t s) {
-    const size_t texels = (size_t)n * n * n;
-    quads3_kernel<<<(unsigned)((texels + 255) / 256), 256, 0, s>>>(vol, n, quads);
-    return cudaGetLastError();
-}
-cudaError_t launch_cells2(const uint32_t* img, int n, uint4* cells, cudaStream_t s) {
-    const size_t texels = (size_t)n * n;
-    cells2_kernel<<<(unsigned)((texels + 255) / 256), 256, 0, s>>>(img, n, cells);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_generate_base(uint32_t seed, NoiseOut o, cudaStream_t s) {
-    const dim3 grid(MT_BASE_N / kTileX, MT_BASE_N / kTileY, MT_BASE_N / kTileZ);
-    gen_base_kernel<<<grid, 256, 0, s>>>(seed, o);
-    return cudaGetLastError();
-}
-cudaError_t launch_generate_detail(uint32_t seed, NoiseOut o, cudaStream_t s) {
-    const unsigned n = MT_DETAIL_N * MT_DETAIL_N * MT_DETAIL_N;
-    gen_detail_kernel<<<(n + 127) / 128, 128, 0, s>>>(seed, o);
-    return cudaGetLastError();
-}
-cudaError_t launch_generate_curl(uint32_t seed, NoiseOut o, cudaStream_t s) {
-    const unsigned n = MT_CURL_N * MT_CURL_N;
-    gen_curl_kernel<<<(n + 127) / 128, 128, 0, s>>>(seed, o);
+cudaError_t launch_generate_volumes(uint32_t seed, NoiseOut base, NoiseOut detail, NoiseOut curl, NoiseOut weather,
+                                    cudaStream_t s) {
+    gen_volumes_kernel<<<kBaseTiles + kWeatherBlocks + kDetailBlocks + kCurlBlocks, kGenThreads, 0, s>>>(
+        seed, base, detail, curl, weather);
     return cudaGetLastError();
 }
 cudaError_t launch_generate_weather(uint32_t seed, NoiseOut o, cudaStream_t s) {
-    const unsigned n = MT_WEATHER_N * MT_WEATHER_N;
-    gen_weather_kernel<<<(n + 127) / 128, 128, 0, s>>>(seed, o);
-    return cudaGetLastError();
-}
-cudaError_t launch_u8_to_16(const uint32_t* src, size_t n, uint2* h16, uint2* b16, cudaStream_t s) {
-    u8_to_16_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, n, h16, b16);
+    gen_weather_kernel<<<kWeatherBlocks, kGenThreads, 0, s>>>(seed, o);
     return cudaGetLastError();
 }
 

@@ -31,3 +31,37 @@ def test_generator_bit_exact_over_seeds(context, oracle, seed):
             assert np.array_equal(got[k], want[k]), k
             assert np.array_equal(half[k], want[k + "_h16"]), k
             assert np.array_equal(bf[k], want[k + "_b16"]), k
+
+
+@pytest.mark.parametrize("changed", [("base",), ("detail",), ("curl",), ("weather",), ("detail", "curl"), KEYS])
+def test_layouts_follow_each_change(context, changed):
+    """Uploading some volumes over generated ones gives the frames of a context
+    that was given all of them, in every storage, and a generated volume's
+    layouts are its own."""
+    rng = np.random.default_rng(11)
+    with context(0) as a, context(0) as b:
+        a.generate_volumes(3)
+        vols = a.download_volumes()
+        new = dict(vols)
+        for k in changed:
+            new[k] = rng.integers(0, 256, vols[k].shape, dtype=np.uint8)
+        a.upload_volumes(**vols)  # bytes for all: the 16-bit texels are the bytes' too
+        a.upload_volumes(**{k: new[k] for k in changed})
+        b.upload_volumes(**new)
+        cam, tm, params, _ = scenes.config_view(6, 64, 36)
+        for storage in (abi.MT_STORAGE_U8, abi.MT_STORAGE_F16, abi.MT_STORAGE_BF16):
+            params.storage = storage
+            frames = []
+            for ctx in (a, b):
+                cur = torch.zeros((36, 64, 4), device="cuda")
+                ctx.render(cam, cam, tm, params, None, cur, None, abi.MT_RENDER_FULL)
+                frames.append(cur.cpu().numpy())
+                got = ctx.download_volumes()
+                assert all(np.array_equal(got[k], new[k]) for k in KEYS)
+            assert_bits_equal(frames[0], frames[1], f"storage {storage}")
+            if storage:
+                got = a.download_volumes_16(storage)
+                for k in KEYS:
+                    c = torch.from_numpy(new[k].astype(np.float32)) / 255.0
+                    want = c.half() if storage == abi.MT_STORAGE_F16 else c.bfloat16()
+                    assert np.array_equal(got[k], want.view(torch.int16).numpy().view(np.uint16)), k
