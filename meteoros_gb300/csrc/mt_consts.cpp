@@ -75,6 +75,8 @@ void make_view_consts(ViewConsts* v, const mt_params& p, const mt_camera_ubo& ca
     rcp(v->r_h, (float)H);
     rcp(v->r_tanx, v->tanx);
     rcp(v->r_tany, v->tany);
+    const float tx = std::fabs(v->tanx), ty = std::fabs(v->tany);
+    v->tame = tx >= 0x1p-30f && tx <= 0x1p30f && ty >= 0x1p-30f && ty <= 0x1p30f ? 1 : 0;
     for (int i = 0; i < 16; ++i) v->ov[i] = cam_old.view[i];
 }
 

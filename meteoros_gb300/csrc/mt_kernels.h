@@ -21,6 +21,7 @@ struct ViewConsts {
     float eye[3], right[3], up[3], ref[3], ec[3], ro[3];
     float jx, jy, tanx, tany, C, Rin;
     float r_w[2], r_h[2], r_tanx[2], r_tany[2];  // {b, RN(1/b)}
+    int32_t tame;  // tanx and tany within 2^30 of 1: see old_uv (mt_render.cu)
     float ov[16];
 };
 

@@ -31,14 +31,17 @@ struct Isect {
 // and ref = eye + look are the same for every pixel: they come in `v`, made
 // on the host by make_view_consts with the same operations (mt_consts.cpp),
 // and each ray computes only its own part.
-MT_HD Ray cast_ray(const ViewConsts& v, f3 eye, float sx, float sy) {
+MT_HD f3 cast_direction(const ViewConsts& v, f3 eye, float sx, float sy) {  // not normalised
     float nx = sx * 2.0f - 1.0f, ny = sy * 2.0f - 1.0f;
     nx = nx + v.jx;
     ny = ny + v.jy;
     const f3 cam_x = (nx * v.tanx) * ld3(v.right);
     const f3 cam_y = (ny * v.tany) * ld3(v.up);
     const f3 pp = ld3(v.ref) + cam_x + cam_y;
-    return Ray{eye, normalize3_r(pp - eye)};
+    return pp - eye;
+}
+MT_HD Ray cast_ray(const ViewConsts& v, f3 eye, float sx, float sy) {
+    return Ray{eye, normalize3_r(cast_direction(v, eye, sx, sy))};
 }
 
 // cloudRayMarch.comp:229-273 (t = length(p - rO) with the normalised rO, as

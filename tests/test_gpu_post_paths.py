@@ -36,3 +36,47 @@ def test_godray_forms_bit_exact(ctx, oracle, size, light):
         ctx.godrays(cam, light, to_dev(mask, torch), to_dev(img, torch), out)
         want = oracle.godrays(cam, np.array(light, np.float32), mask, img)
         assert_bits_equal(out.cpu().numpy(), want, f"{size} yaw {yaw}")
+
+
+# The previous camera's uv checks three denominators instead of eleven quotients
+# and takes the checked routine where one is out of range: cameras that look
+# across and away from the shell hits, fields of view inside and outside the
+# range, images without an interior for the history's filter.
+@pytest.mark.parametrize("size", [(1, 1), (2, 2), (5, 3), (66, 37)])
+@pytest.mark.parametrize("case", ["turned", "across", "away", "up", "narrow", "narrowest", "wide", "widest"])
+def test_previous_uv_forms_bit_exact(vctx, oracle, vol7, size, case):
+    w, h = size
+    yaw, pitch, tan = {"turned": (1.5, 15.0, None), "across": (90.0, 0.0, None), "away": (180.0, -15.0, None),
+                       "up": (0.0, 89.9, None), "narrow": (0.5, 15.0, 2.0**-29), "narrowest": (0.5, 15.0, 2.0**-31),
+                       "wide": (0.5, 15.0, 2.0**29), "widest": (0.5, 15.0, 2.0**31)}[case]
+    cam = scenes.look((0.0, 100.0, 0.0), 0.0, 15.0, 60.0, w, h)
+    old = scenes.look((0.0, 100.0, 0.0), yaw, pitch, 60.0, w, h)
+    if tan is not None:
+        cam.tan_fov_by_2[0], cam.tan_fov_by_2[1] = tan, tan
+    _, tm, params, _ = scenes.config_view(2, w, h)
+    tm.frame_count_mod16 = 7
+    rng = np.random.default_rng(w + h)
+    prev, hist = (rng.random((h, w, 4), dtype=np.float32) for _ in range(2))
+    want, wmask, _ = oracle.render(vol7, cam, old, tm, params, prev, w, h, 0)
+    cur = torch.zeros((h, w, 4), device="cuda")
+    vctx.render(cam, old, tm, params, to_dev(prev, torch), cur)
+    repro = np.isnan(wmask)  # not marched
+    got = cur.cpu().numpy()
+    assert_bits_equal(got[repro], want[repro], "reprojected")
+    out = torch.zeros((h, w, 4), device="cuda")
+    vctx.txaa(cam, old, tm, params, cur, to_dev(hist, torch), out)
+    assert_bits_equal(out.cpu().numpy(), oracle.txaa(cam, old, tm, params, got, hist), "txaa")
+    frame, resolved = torch.zeros_like(cur), torch.zeros_like(cur)
+    vctx.render_frame(cam, old, tm, params, to_dev(prev, torch), frame, to_dev(hist, torch), resolved)
+    assert_bits_equal(frame.cpu().numpy(), got, "frame")
+    assert_bits_equal(resolved.cpu().numpy(), out.cpu().numpy(), "resolved")
+
+
+@pytest.fixture(scope="module")
+def vctx(lib):
+    from meteoros_gb300.renderer import Context
+
+    c = Context(0)
+    c.generate_volumes(7)
+    yield c
+    c.close()
