@@ -154,6 +154,9 @@ struct BatchTile {
     int32_t nrx, nry;  // the view's ray grid: pixels (full) or 4x4 blocks (checkerboard)
 };
 
+// Branches of a batch's graph that its reprojections are spread over.
+constexpr int kBatchBranches = 4;
+
 // A batch of views marched by one persistent launch: every CTA takes tiles
 // from `counter` (zeroed before the launch) until all are done.
 struct BatchArgs {

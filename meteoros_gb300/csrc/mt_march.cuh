@@ -563,7 +563,9 @@ template <int S> cudaError_t launch_batch_storage(const BatchArgs& b, int lanes,
     }
     switch (lanes) {
         case 1: march_batch_kernel<1, S, kTame><<<blocks, 128, 0, s>>>(b); break;
+        case 2: march_batch_kernel<2, S, kTame><<<blocks, 128, 0, s>>>(b); break;
         case 4: march_batch_kernel<4, S, kTame><<<blocks, 128, 0, s>>>(b); break;
+        case 32: march_batch_kernel<32, S, kTame><<<blocks, 128, 0, s>>>(b); break;
         case 16: march_batch_kernel<16, S, kTame><<<blocks, 128, 0, s>>>(b); break;
         default: march_batch_kernel<8, S, kTame><<<blocks, 128, 0, s>>>(b); break;
     }
@@ -576,7 +578,9 @@ template <int S> int batch_blocks_storage(int device, int lanes) {
     auto occupancy = [&](auto kernel) { cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0); };
     switch (lanes) {
         case 1: occupancy(march_batch_kernel<1, S, kTame>); break;
+        case 2: occupancy(march_batch_kernel<2, S, kTame>); break;
         case 4: occupancy(march_batch_kernel<4, S, kTame>); break;
+        case 32: occupancy(march_batch_kernel<32, S, kTame>); break;
         case 16: occupancy(march_batch_kernel<16, S, kTame>); break;
         default: occupancy(march_batch_kernel<8, S, kTame>); break;
     }
