@@ -21,6 +21,8 @@
 
 #include "mt_kernels.h"
 
+static_assert(MT_BASE_N == 1 << 7 && MT_DETAIL_N == 1 << 5, "the TGA decode's slice sizes");
+
 struct mt_ctx {
     int device = 0;
     std::string err;
@@ -403,7 +405,7 @@ MT_API mt_status mt_decode_tga_volume(mt_ctx* ctx, int volume, const uint8_t* co
         if (w != n || h != n)
             return fail(ctx, MT_ERR_INVALID_ARG, "slice %d is %dx%d, the volume's slices are %dx%d", z, w, h, n, n);
         table[(size_t)z] = mt::TgaSlice{(long long)total, (long long)sz};
-        total += sz;
+        total += (sz + 15) / 16 * 16;
         max_size = std::max(max_size, sz);
     }
     mt_status st;
@@ -420,7 +422,7 @@ MT_API mt_status mt_decode_tga_volume(mt_ctx* ctx, int volume, const uint8_t* co
     if (e == cudaSuccess) e = cudaMemcpy(d_blob, blob.data(), total, cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(d_table, table.data(), table.size() * sizeof(mt::TgaSlice), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = mt::launch_tga_decode(d_blob, d_table, n, max_size, vol, n, n, s);
+    if (e == cudaSuccess) e = mt::launch_tga_decode(d_blob, d_table, n, max_size, vol, volume == MT_VOLUME_BASE ? 7 : 5, s);
     const mt::LayoutJob job = volume == MT_VOLUME_BASE ? base_job(ctx) : detail_job(ctx);
     if (e == cudaSuccess) e = mt::launch_layouts(&job, 1, true, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -189,7 +189,8 @@ struct TonemapArgs {
     int32_t width, height;
 };
 
-// One TGA file of a volume's slice stack, inside the concatenated upload.
+// One TGA file of a volume's slice stack, inside the packed upload: at a
+// 16-byte offset, the upload readable to the next one past its end.
 struct TgaSlice {
     long long offset;
     long long size;
@@ -234,8 +235,9 @@ cudaError_t launch_march_f16(const MarchArgs& a, cudaStream_t s, long long rays)
 cudaError_t launch_march_bf16(const MarchArgs& a, cudaStream_t s, long long rays);
 cudaError_t launch_txaa(const TxaaArgs& a, cudaStream_t s, const cudaEvent_t* ev);
 cudaError_t launch_godrays(const GodrayArgs& a, cudaStream_t s);
+// Slices of 2^log2n x 2^log2n pixels.
 cudaError_t launch_tga_decode(const unsigned char* blob, const TgaSlice* slices, int n_slices, size_t max_size,
-                              uint32_t* vol, int W, int H, cudaStream_t s);
+                              uint32_t* vol, int log2n, cudaStream_t s);
 cudaError_t launch_tonemap(const TonemapArgs& a, cudaStream_t s);
 // The raymarch, then reprojection fused with TXAA (a.history -> a.out).
 cudaError_t launch_frame(const MarchArgs& a, cudaStream_t s, const LaunchEvents* ev, const ForkJoin* fj);

@@ -65,3 +65,33 @@ def test_layouts_follow_each_change(context, changed):
                     c = torch.from_numpy(new[k].astype(np.float32)) / 255.0
                     want = c.half() if storage == abi.MT_STORAGE_F16 else c.bfloat16()
                     assert np.array_equal(got[k], want.view(torch.int16).numpy().view(np.uint16)), k
+
+
+@pytest.mark.parametrize("kind", ["literal", "runs", "mixed", "single", "truncated"])
+def test_tga_packet_shapes(context, oracle, kind):
+    """Packets of 128, of 1 and of every length between, literal and run, files
+    cut off at every kind of byte, sizes that are no multiple of 16."""
+    import ctypes as C
+
+    n = abi.MT_DETAIL_N
+    rng = np.random.default_rng(5)
+    files = []
+    for z in range(n):
+        head = bytearray([z % 3, 0, 10, 0, 0, 0, 0, 0, 0, 0, 0, 0, n, 0, n, 0, 32 if z % 2 else 24, 32 * (z % 4 == 1)])
+        body, left = bytearray(rng.integers(0, 256, z % 3, dtype=np.uint8).tobytes()), n * n
+        while left > 0:
+            length = {"literal": 128, "runs": 128, "single": 1}.get(kind, int(rng.integers(1, 129)))
+            run = kind == "runs" or (kind != "literal" and rng.random() < 0.5)
+            px = 1 if run else length
+            body.append((128 if run else 0) | (length - 1))
+            body += rng.integers(0, 256, px * (4 if z % 2 else 3), dtype=np.uint8).tobytes()
+            left -= length
+        data = bytes(head + body)
+        files.append(data[:18 + z * 61 % (len(data) - 18)] if kind == "truncated" else data)
+    want = np.stack([oracle.decode_tga(f) for f in files])
+    arr = (C.c_void_p * n)(*[C.cast(C.c_char_p(f), C.c_void_p) for f in files])
+    sizes = (C.c_size_t * n)(*[len(f) for f in files])
+    with context(0) as ctx:
+        ctx.generate_volumes(1)
+        assert ctx.lib.mt_decode_tga_volume(ctx.handle, abi.MT_VOLUME_DETAIL, arr, sizes, n, None) == abi.MT_OK
+        assert np.array_equal(ctx.download_volumes()["detail"], want)
