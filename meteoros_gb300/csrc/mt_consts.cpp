@@ -110,7 +110,9 @@ namespace {
 //     y stays half an Earth radius above the centre's: the eye's does, and dir.y
 //     + jitter.y is positive), so products below 2^-100 round away.  Heights'
 //     gradients and energies see 0 or differences of numbers near 1.
-// Other frames are marched with the checks (kGeneral).
+// The same bounds settle the special cases of the RGBA8 form's reciprocals, roots
+// and clamps (kExact, mt_march.cuh).  Other frames are marched with the checks
+// (kGeneral).
 bool frame_is_tame(const Frame& f, const mt_params& p, const float jitter[16][3]) {
     const double kFar = 0x1p30, kSmall = 0x1p-10, kScale = 0x1p-20;
     auto len = [](const float v[3]) {
@@ -123,6 +125,12 @@ bool frame_is_tame(const Frame& f, const mt_params& p, const float jitter[16][3]
     if (p.coverage_mode == 1) ok = ok && p.weather_scale >= kScale && p.weather_scale <= kFar;
     for (int i = 0; i < 16; ++i)
         for (int c = 0; c < 3; ++c) ok = ok && std::fabs(jitter[i][c]) <= 0.05f;
+    // a constant coverage, and its remap's width, 0 or within 2^30 of 1 (a weather
+    // map's are 0 or at least 2^-32); t below 2^24 - 16
+    if (p.coverage_mode == 0)
+        for (const double c : {std::fabs((double)p.coverage), std::fabs((double)(1.0f - p.coverage))})
+            ok = ok && (c == 0.0 || (c >= 0x1p-30 && c <= 0x1p30));
+    ok = ok && 1.1 * (len(f.ec) + f.Rout + std::fmax(len(f.sh32_o[0]), len(f.sh32_o[1]))) < 0x1p24 - 16.0;
     return ok;  // false for NaN
 }
 

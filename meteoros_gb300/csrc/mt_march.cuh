@@ -41,6 +41,13 @@ template <class P> struct Vol16 {
 template <> struct Vol<MT_STORAGE_F16> : Vol16<__half2> {};
 template <> struct Vol<MT_STORAGE_BF16> : Vol16<__nv_bfloat162> {};
 
+// The RGBA8 form's tame frames: every special case of the density path's
+// arithmetic -- operands of the reciprocals, roots and quotients far from 1, NaN
+// in the clamps -- is settled by Frame::tame, so it runs on rcp_core, sqrt_core
+// and saturating instructions, value for value the shader's.  (The 16-bit
+// forms' compiler settings have approximations there already.)
+template <int S, bool TAME> constexpr bool kExact = TAME && S == MT_STORAGE_U8;
+
 struct Weather {
     float lo, mul, type;
     float hgrad;  // height gradient at the primary sample, shared by its light samples
@@ -74,14 +81,22 @@ MT_HD Weather weather_at(const mt_params& p, const Frame& F, const Tex<S>& tx, f
         w.mul = wd.x;
         w.type = wd.z;
     }
-    w.r_lo = Rcp{1.0f - w.lo, __fdividef(1.0f, 1.0f - w.lo)};
+    w.r_lo = Rcp{1.0f - w.lo, kExact<S, TAME> ? rcp_approx(1.0f - w.lo) : __fdividef(1.0f, 1.0f - w.lo)};
     return w;
 }
 
 // cloudRayMarch.comp:499-540
-template <int S>
+template <int S, bool TAME>
 MT_HD float sample_low_frequency(const mt_params& p, const Tex<S>& tx, f3 point, float relH, const Weather& wt) {
     f4v n = Vol<S>::template tex3<MT_BASE_N>(tx.base, point);
+    if (kExact<S, TAME>) {
+        const float fbm = __saturatef((n.y * 0.625f) + (n.z * 0.25f) + (n.w * 0.125f));
+        const float lo = fbm - 0.9f;
+        float shape = __saturatef(div_core(n.x - lo, 1.0f - lo));
+        if (p.height_gradient) shape = shape * wt.hgrad;
+        // 0 / 0, where the threshold is 1, saturates to 0: as empty as its NaN
+        return __saturatef(div_core(fminf(fmaxf(shape, wt.lo), 1.0f) - wt.lo, wt.r_lo.b)) * wt.mul;
+    }
     float fbm = (n.y * 0.625f) + (n.z * 0.25f) + (n.w * 0.125f);
     fbm = gclamp(fbm, 0.0f, 1.0f);
     float baseCloud = remap_clamped(n.x, (fbm - 0.9f), 1.0f, 0.0f, 1.0f);
@@ -141,12 +156,13 @@ MT_HD float2 sample_light_pair(const mt_params& p, const uint4* base, f3 s0, f3 
 // cloudRayMarch.comp:542-563.  The texture part is the same for the primary
 // erosion (:645) and the six cone-light erosions (:665): all are evaluated at
 // the primary sample point with the primary height, so it is computed once.
-template <int S> MT_HD float erosion_modifier(const Tex<S>& tx, f3 point, float h) {
+template <int S, bool EXACT> MT_HD float erosion_modifier(const Tex<S>& tx, f3 point, float h) {
     f4v curl = Vol<S>::template tex2<MT_CURL_N>(tx.curl, point.x, point.y);
     point.x = point.x + (curl.x * (1.0f - h)) * 0.5f;
     point.y = point.y + (curl.y * (1.0f - h)) * 0.5f;
     f4v hf = Vol<S>::template tex3<MT_DETAIL_N>(tx.detail, point);
     float hfbm = (hf.x * 0.625f) + (hf.y * 0.25f) + (hf.z * 0.125f);
+    if (EXACT) return __saturatef(gmix(hfbm, 1.0f - hfbm, __saturatef(h * 2.0f)));
     return gclamp(gmix(hfbm, 1.0f - hfbm, gclamp(h * 2.0f, 0.0f, 1.0f)), 0.0f, 1.0f);
 }
 // Per-ray constants of cloudRayMarch.comp:565-624, shared by every step (the
@@ -185,7 +201,12 @@ constexpr int kInCloud = 16;
 
 // How a march is compiled: for tame frames (Frame::tame: no range checks on the
 // steps' quotients), for every frame, and for every frame with the per-ray trace.
-constexpr int kTame = 0, kGeneral = 1, kTraced = 2;
+// kBatch is kTame as the batch kernel takes it: its views' constants come from
+// memory and press on the registers, so the library's square root and the light
+// samples three a turn do better there (20-view batch 9.54 / 8.05 -> 9.31 / 7.86 ms by
+// view, 24 sessions 1.59 / 1.38 -> 1.55 / 1.34; frames lose 1 %).
+constexpr int kTame = 0, kGeneral = 1, kTraced = 2, kBatch = 3;
+template <int MODE> constexpr bool kIsTame = MODE == kTame || MODE == kBatch;
 
 // One iteration of the march loop body (cloudRayMarch.comp:629-678) at
 // parameter t, up to the accumulation: everything that does not depend on the
@@ -193,14 +214,17 @@ constexpr int kTame = 0, kGeneral = 1, kTraced = 2;
 template <int S, int MODE>
 MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, const mt_time_ubo& tm,
                         const float (*jitter)[3], const RayConsts& rc, float t) {
-    constexpr bool TAME = MODE == kTame, TR = MODE == kTraced;
+    constexpr bool TAME = kIsTame<MODE>, TR = MODE == kTraced, EXACT = kExact<S, TAME>;
     StepOut o{0, 0.0f, 0.0f};
-    const int _index = f2i(gmod((float)(tm.frame_count_mod16 + f2i(t)), 16.0f));
-    if (TR) o.code = _index & 15;
-    const float* j = jitter[_index & 15];  // _index is in 0..15 for every finite t
+    // int(mod(float(frame + int(t)), 16)), 0..15 for every finite t; in a tame
+    // frame (t below 2^24 - 16) the low four bits of the whole number
+    const int step = tm.frame_count_mod16 + f2i(t);
+    const int _index = (TAME ? step : f2i(gmod((float)step, 16.0f))) & 15;
+    if (TR) o.code = _index;
+    const float* j = jitter[_index];
     f3 jd = rc.dir + f3{j[0], j[1], j[2]};
     f3 pos = ld3(F.eye) + t * jd;
-    const float relH = relative_height<TAME>(F, pos, ld3(F.ec), rc.lenInner, rc.dir, ld3(F.eye));
+    const float relH = relative_height<TAME, EXACT, EXACT && MODE == kTame>(F, pos, ld3(F.ec), rc.lenInner, rc.dir, ld3(F.eye));
     // Empty steps, found before anything is fetched for them (results unchanged;
     // of the benchmark views' executed steps 12 % are too high, 6 % have no
     // gradient otherwise and 25 % only a gradient below the threshold.  960x540
@@ -210,7 +234,7 @@ MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, co
     Weather wt = weather_at<S, TAME>(p, F, tx, pos, ld3(F.ec));
     // (the 16-bit forms keep its check: without it their compiler settings
     // contract its blends another way, which moves their results by roundings)
-    if (p.height_gradient) wt.hgrad = height_gradient<TAME && S == MT_STORAGE_U8>(relH, wt.type);
+    if (p.height_gradient) wt.hgrad = height_gradient<EXACT, EXACT>(relH, wt.type);
     // ... a zero height gradient or zero coverage makes the density 0 (or NaN
     // when the coverage is 0), never > 0 ...
     if ((p.height_gradient && wt.hgrad == 0.0f) || wt.mul == 0.0f) return o;
@@ -223,11 +247,11 @@ MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, co
     sp = rdiv3_step<TAME>(sp, F.r_period);
     sp = sp + ((relH * ld3(F.skew)) * p.cloud_top_offset) * 0.009f;
     sp = sp + ld3(F.wind_t);
-    float baseDensity = sample_low_frequency<S>(p, tx, sp, relH, wt) * 0.380f;
+    float baseDensity = sample_low_frequency<S, TAME>(p, tx, sp, relH, wt) * 0.380f;
     if (baseDensity > 0.0f) {
-        const Erosion ero = make_erosion(erosion_modifier<S>(tx, sp, relH));
+        const Erosion ero = make_erosion<EXACT>(erosion_modifier<S, EXACT>(tx, sp, relH));
         o.code |= kInCloud;
-        o.hfd = erode(baseDensity * 1.4f, ero);
+        o.hfd = erode<EXACT>(baseDensity * 1.4f, ero);
         float dl = 0.0f;
         // The six cone-light samples (colour only: see sample_light), unrolled in
         // the FP32-filtered forms: the offsets koff[i] stay in registers instead
@@ -246,7 +270,8 @@ MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, co
             return f3{__fadd_rn(prel.x, k.x), __fadd_rn(prel.y, k.y), __fadd_rn(prel.z, k.z)};
         };
         if constexpr (S != MT_STORAGE_F16) {
-#pragma unroll
+            constexpr int kTurn = MODE == kBatch ? 3 : 6;
+#pragma unroll kTurn
             for (int i = 0; i < 6; ++i) {
                 const float cbl = sample_light<S>(p, tx, light_point(i), wt);
                 if (cbl > 0.0f) {
@@ -270,7 +295,7 @@ MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, co
                 }
             }
         }
-        o.E = light_energy<TAME>(relH, dl, baseDensity, rc.HG_light, rc.cos_q, 5.0f);
+        o.E = light_energy<TAME, EXACT>(relH, dl, baseDensity, rc.HG_light, rc.cos_q, 5.0f);
     }
     return o;
 }
@@ -562,12 +587,12 @@ template <int S> cudaError_t launch_batch_storage(const BatchArgs& b, int lanes,
         return cudaGetLastError();
     }
     switch (lanes) {
-        case 1: march_batch_kernel<1, S, kTame><<<blocks, 128, 0, s>>>(b); break;
-        case 2: march_batch_kernel<2, S, kTame><<<blocks, 128, 0, s>>>(b); break;
-        case 4: march_batch_kernel<4, S, kTame><<<blocks, 128, 0, s>>>(b); break;
-        case 32: march_batch_kernel<32, S, kTame><<<blocks, 128, 0, s>>>(b); break;
-        case 16: march_batch_kernel<16, S, kTame><<<blocks, 128, 0, s>>>(b); break;
-        default: march_batch_kernel<8, S, kTame><<<blocks, 128, 0, s>>>(b); break;
+        case 1: march_batch_kernel<1, S, kBatch><<<blocks, 128, 0, s>>>(b); break;
+        case 2: march_batch_kernel<2, S, kBatch><<<blocks, 128, 0, s>>>(b); break;
+        case 4: march_batch_kernel<4, S, kBatch><<<blocks, 128, 0, s>>>(b); break;
+        case 32: march_batch_kernel<32, S, kBatch><<<blocks, 128, 0, s>>>(b); break;
+        case 16: march_batch_kernel<16, S, kBatch><<<blocks, 128, 0, s>>>(b); break;
+        default: march_batch_kernel<8, S, kBatch><<<blocks, 128, 0, s>>>(b); break;
     }
     return cudaGetLastError();
 }
@@ -577,12 +602,12 @@ template <int S> int batch_blocks_storage(int device, int lanes) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     auto occupancy = [&](auto kernel) { cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0); };
     switch (lanes) {
-        case 1: occupancy(march_batch_kernel<1, S, kTame>); break;
-        case 2: occupancy(march_batch_kernel<2, S, kTame>); break;
-        case 4: occupancy(march_batch_kernel<4, S, kTame>); break;
-        case 32: occupancy(march_batch_kernel<32, S, kTame>); break;
-        case 16: occupancy(march_batch_kernel<16, S, kTame>); break;
-        default: occupancy(march_batch_kernel<8, S, kTame>); break;
+        case 1: occupancy(march_batch_kernel<1, S, kBatch>); break;
+        case 2: occupancy(march_batch_kernel<2, S, kBatch>); break;
+        case 4: occupancy(march_batch_kernel<4, S, kBatch>); break;
+        case 32: occupancy(march_batch_kernel<32, S, kBatch>); break;
+        case 16: occupancy(march_batch_kernel<16, S, kBatch>); break;
+        default: occupancy(march_batch_kernel<8, S, kBatch>); break;
     }
     return (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
 }

@@ -120,11 +120,12 @@ MT_HD float remap_clamped(float v, float omin, float omax, float nmin, float nma
 // cloudRayMarch.comp:171-186
 // lenInner = length(startPos - eye) is the same for every step of a ray; the
 // raymarch passes it in precomputed.
-template <bool TAME>
+template <bool TAME, bool CORE_RCP, bool CORE_ROOT>
 MT_HD float relative_height(const Frame& F, f3 point, f3 ec, float lenInner, f3 rayDir, f3 eye) {
-    float lenCam = length3(point - eye);
-    const f3 up = point - ec;
-    f3 p2e = rdiv3_step<TAME>(up, make_rcp(length3(up)));
+    const f3 toCam = point - eye, up = point - ec;
+    const float lenCam = CORE_ROOT ? sqrt_core(dot3(toCam, toCam)) : length3(toCam);
+    const float lenUp = CORE_ROOT ? sqrt_core(dot3(up, up)) : length3(up);
+    f3 p2e = rdiv3_step<TAME>(up, CORE_RCP ? Rcp{lenUp, rcp_core(lenUp)} : make_rcp(lenUp));
     float cosTheta = dot3(rayDir, p2e);
     float num = fabsf(cosTheta * (lenCam - lenInner));
     return rdiv_step<TAME>(num, F.r_thick);
@@ -146,13 +147,21 @@ static __device__ __noinline__ HgQuot hg_quotients_exceptional(float h) {
 
 // cloudRayMarch.comp:475-487.  The remaps' four quotients share one range
 // check (rdiv_core; all four redone by rdiv when any falls outside it).
-template <bool TAME> MT_HD float height_gradient(float h, float type) {
-    h = gclamp(h, 0.0f, 1.0f);
+// EXACT: the same values from saturating and min/max instructions, which differ
+// from the shader's selects in the sign of a zero only (no operand is NaN).
+template <bool TAME, bool EXACT> MT_HD float height_gradient(float h, float type) {
+    h = EXACT ? __saturatef(h) : gclamp(h, 0.0f, 1.0f);
     HgQuot q{rdiv_core(h - 0.0f, MT_RCP(0.0f, 0.25f)), rdiv_core(h - 0.3f, MT_RCP(0.3f, 0.65f)),
              rdiv_core(h - 0.0f, MT_RCP(0.0f, 0.1f)), rdiv_core(h - 0.2f, MT_RCP(0.2f, 0.3f))};
     if (!TAME && !(rdiv_in_range(q.q1) & rdiv_in_range(q.q2) & rdiv_in_range(q.q3) & rdiv_in_range(q.q4)))
         q = hg_quotients_exceptional(h);
     // remap(h, omin, omax, nmin, nmax) = nmin + q * (nmax - nmin)
+    if (EXACT) {
+        const float strato = fmaxf(0.0f, q.q1 * (1.0f - q.q2)), stratus = fmaxf(0.0f, q.q3 * (1.0f - q.q4));
+        const float a = gmix(stratus, strato, __saturatef(type * 2.0f));
+        const float b = gmix(strato, stratus, __saturatef((type - 0.5f) * 2.0f));
+        return gmix(a, b, type);
+    }
     float stratocumulus = gmax(0.0f, (0.0f + (q.q1 * (1.0f - 0.0f))) * (1.0f + (q.q2 * (0.0f - 1.0f))));
     float stratus = gmax(0.0f, (0.0f + (q.q3 * (1.0f - 0.0f))) * (1.0f + (q.q4 * (0.0f - 1.0f))));
     float a = gmix(stratus, stratocumulus, gclamp(type * 2.0f, 0.0f, 1.0f));
@@ -165,13 +174,16 @@ struct Erosion {
     Rcp r;     // {1 - lo, ~1/(1 - lo)}: the width (b, exact division) and an
                // approximate reciprocal for the light samples (y)
 };
-MT_HD Erosion make_erosion(float modifier) {
+template <bool EXACT> MT_HD Erosion make_erosion(float modifier) {
     Erosion e;
     e.lo = modifier * 0.005f;
-    e.r = Rcp{1.0f - e.lo, __fdividef(1.0f, 1.0f - e.lo)};
+    e.r = Rcp{1.0f - e.lo, EXACT ? rcp_approx(1.0f - e.lo) : __fdividef(1.0f, 1.0f - e.lo)};
     return e;
 }
-MT_HD float erode(float baseCloud, const Erosion& e) { return 0.0f + (((baseCloud - e.lo) / e.r.b) * (1.0f - 0.0f)); }
+template <bool EXACT> MT_HD float erode(float baseCloud, const Erosion& e) {
+    if (EXACT) return div_core(baseCloud - e.lo, e.r.b);
+    return 0.0f + (((baseCloud - e.lo) / e.r.b) * (1.0f - 0.0f));
+}
 
 // cloudRayMarch.comp:295-306.  The phase weights the light energy and the
 // sky, colour only: pow in the special-function unit's form (see
@@ -188,7 +200,16 @@ MT_HD float henyey_greenstein(float c, float e) {
 // which is how GLSL defines pow's precision: they differ from the correctly
 // rounded values by tens of ulp at most.  The light energy reaches colour
 // only, never the accumulated density, the control flow or the god-ray mask.
-template <bool TAME> MT_HD float light_energy(float h, float dl, float ds, float phase, float cos_q, float brightness) {
+template <bool TAME, bool EXACT>
+MT_HD float light_energy(float h, float dl, float ds, float phase, float cos_q, float brightness) {
+    if (EXACT) {  // the same operations, special-function forms and clamps as single instructions
+        const float primary = exp_ftz(-dl);
+        const float att = fmaxf(primary + (cos_q * (primary * 0.25f - primary)), primary);
+        const float e = fminf(fmaxf(remap_r<true>(h * 0.125f, 0.3f, MT_RCP(0.3f, 0.85f), 0.5f, 2.0f), 0.5f), 2.0f);
+        const float v = fminf(fmaxf(remap_r<true>(h * 1.5f, 0.07f, MT_RCP(0.07f, 0.34f), 0.1f, 1.0f), 0.1f), 1.0f);
+        const float in_scatter = (0.05f + pow_ftz(ds, e)) * pow_ftz(v, 0.8f);
+        return att * primary * in_scatter * phase * brightness;
+    }
     const float primary = __expf(-dl);
     const float secondary = primary;  // exp(-dl) twice in the reference (:334, :340)
     float att = gmax(secondary + (cos_q * (secondary * 0.25f - secondary)), primary);

@@ -152,3 +152,12 @@ def test_early_exit_at_every_limit(ctx, oracle, vol7, lanes, limit):
     ctx.set_tuning(march_lanes=lanes)
     check_density(oracle, vol7, ctx, params, cam, tm)
     ctx.set_tuning(march_lanes=0)
+
+
+@pytest.mark.parametrize("coverage", [2.0**-29, 2.0**-31, 1.0 - 2.0**-24, 2.0**29, 2.0**31, -2.0**20])
+def test_coverage_bounds_equal_oracle(ctx, oracle, vol7, coverage):
+    """Constant coverages on either side of the bounds under which the density
+    path drops its special cases."""
+    cam, tm, params, _ = scenes.config_view(3, W, H)
+    params.coverage_mode, params.coverage, params.height_gradient = 0, coverage, 1
+    check_density(oracle, vol7, ctx, params, cam, tm)
