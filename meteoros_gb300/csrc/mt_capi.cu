@@ -52,9 +52,11 @@ struct mt_ctx {
     int march_order = 0;                      // ray rows: 0 bottom to top, 1 top to bottom
     int batch_order = 0;                      // mt_render_batch tile rows: 0 bottom to top, 1 top to bottom
     int fused_resolve = 0;                    // mt_render_frame: reprojection fused with TXAA
-    // mt_decode_tga_volume: the slice table and the packed files, pinned and on
-    // the device; kept for the next volume (at most kTgaCapacity bytes each)
+    // mt_decode_tga_volume: two pinned pieces that the slice table and the files
+    // are packed into in turn, and the whole on the device; kept for the next
+    // volume (2 MiB, and at most kTgaCapacity bytes)
     uint8_t* tga_host = nullptr;
+    cudaEvent_t tga_sent[2] = {nullptr, nullptr};
     uint8_t* tga_dev = nullptr;
     size_t tga_bytes = 0;
     // mt_render_batch
@@ -186,19 +188,20 @@ mt::LayoutJob weather_job(mt_ctx* c, int slot) {
 // A volume's slice table, then its files at 16-byte offsets, readable to the
 // next one past the last.
 constexpr size_t kTgaTableBytes = MT_BASE_N * sizeof(mt::TgaSlice);
-constexpr size_t kTgaSendBytes = 1 << 20;
+constexpr size_t kTgaPiece = 1 << 20;  // holds the table and any slice
+static_assert(kTgaPiece >= kTgaTableBytes + MT_TGA_MAX_SLICE_BYTES + 16, "a piece holds a slice");
 constexpr size_t kTgaCapacity = kTgaTableBytes + (size_t)MT_BASE_N * (MT_TGA_MAX_SLICE_BYTES + 16);
 
 mt_status ensure_tga_buffers(mt_ctx* ctx, size_t bytes) {
+    if (!ctx->tga_host) MT_CUDA(ctx, cudaHostAlloc((void**)&ctx->tga_host, 2 * kTgaPiece, cudaHostAllocDefault));
+    for (cudaEvent_t& e : ctx->tga_sent)
+        if (!e) MT_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     if (bytes <= ctx->tga_bytes) return MT_OK;
     // a quarter more than asked for, so that the next scene's files fit too
-    const size_t cap = std::min(std::max(bytes + bytes / 4, (size_t)1 << 20), kTgaCapacity);
-    cudaFreeHost(ctx->tga_host);
+    const size_t cap = std::min(std::max(bytes + bytes / 4, kTgaPiece), kTgaCapacity);
     cudaFree(ctx->tga_dev);
-    ctx->tga_host = nullptr;
     ctx->tga_dev = nullptr;
     ctx->tga_bytes = 0;
-    MT_CUDA(ctx, cudaHostAlloc((void**)&ctx->tga_host, cap, cudaHostAllocDefault));
     MT_CUDA(ctx, cudaMalloc((void**)&ctx->tga_dev, cap));
     ctx->tga_bytes = cap;
     return MT_OK;
@@ -346,6 +349,8 @@ MT_API void mt_destroy(mt_ctx* ctx) {
     cudaFree(ctx->stats);
     cudaFreeHost(ctx->tga_host);
     cudaFree(ctx->tga_dev);
+    for (cudaEvent_t e : ctx->tga_sent)
+        if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->ev)
         if (e) cudaEventDestroy(e);
     for (int k = 0; k < 2; ++k) {
@@ -440,24 +445,32 @@ MT_API mt_status mt_decode_tga_volume(mt_ctx* ctx, int volume, const uint8_t* co
     if ((st = bind_device(ctx)) != MT_OK) return st;
     if ((st = ensure_volumes(ctx)) != MT_OK) return st;
     if ((st = ensure_tga_buffers(ctx, kTgaTableBytes + total)) != MT_OK) return st;
-    // Table and files packed into pinned memory, sent a megabyte at a time while
-    // the next one is packed, on the default stream: like a synchronous copy it
-    // waits for what blocking streams still read.  (A zeroed vector, a pageable
-    // copy of it and two device buffers per call: 900 us for the base volume's 8.4
-    // MB, now 430, the packing.)
+    // Table and files packed into pinned memory, a piece while the last one is
+    // sent, on the default stream: like a synchronous copy it waits for what
+    // blocking streams still read.  (A zeroed vector, a pageable copy of it and
+    // two device buffers per call: 900 us for the base volume's 8.4 MB, now 430,
+    // the packing.)
     cudaStream_t s = (cudaStream_t)stream;
-    std::memcpy(ctx->tga_host, table.data(), table.size() * sizeof(mt::TgaSlice));
-    uint8_t* files_host = ctx->tga_host + kTgaTableBytes;
-    size_t sent = 0;
     cudaError_t e = cudaSuccess;
+    std::memcpy(ctx->tga_host, table.data(), table.size() * sizeof(mt::TgaSlice));
+    size_t begin = 0, end = kTgaTableBytes;  // of the piece, in the whole
+    int piece = 0;
     for (int z = 0; e == cudaSuccess && z < n; ++z) {
-        std::memcpy(files_host + table[(size_t)z].offset, files[z], sizes[z]);
-        const size_t packed = kTgaTableBytes + (size_t)table[(size_t)z].offset + sizes[z];
-        if (packed - sent >= kTgaSendBytes || z == n - 1) {
-            e = cudaMemcpyAsync(ctx->tga_dev + sent, ctx->tga_host + sent, packed - sent, cudaMemcpyHostToDevice, 0);
-            sent = packed;
+        const size_t at = kTgaTableBytes + (size_t)table[(size_t)z].offset;
+        if (at + sizes[z] - begin > kTgaPiece) {
+            uint8_t* host = ctx->tga_host + (size_t)(piece & 1) * kTgaPiece;
+            e = cudaMemcpyAsync(ctx->tga_dev + begin, host, end - begin, cudaMemcpyHostToDevice, 0);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->tga_sent[piece & 1], 0);
+            begin = at;
+            ++piece;
+            if (e == cudaSuccess && piece >= 2) e = cudaEventSynchronize(ctx->tga_sent[piece & 1]);
         }
+        std::memcpy(ctx->tga_host + (size_t)(piece & 1) * kTgaPiece + (at - begin), files[z], sizes[z]);
+        end = at + sizes[z];
     }
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(ctx->tga_dev + begin, ctx->tga_host + (size_t)(piece & 1) * kTgaPiece, end - begin,
+                            cudaMemcpyHostToDevice, 0);
     if (s || e != cudaSuccess) {  // the default stream orders itself; after a failure copies may be in flight
         const cudaError_t ec = cudaStreamSynchronize(0);
         if (e == cudaSuccess) e = ec;
