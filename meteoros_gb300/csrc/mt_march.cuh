@@ -368,16 +368,21 @@ MT_HD f3 ray_march_group(const mt_params& p, const Frame& F, const Tex<S>& tx, c
         } else if constexpr (G <= 4) {
 #pragma unroll
             for (int k = 0; k < G; ++k) {
-                if (!__shfl_sync(gmask, valid, k, G)) {
+                // one shuffle for whether the step exists and what it is; its two
+                // values only where it applies them (1080p frame 202 / 167 ->
+                // 201 / 165 us by view, 480x270 full frame 140 / 94 -> 139 / 89)
+                const int code = __shfl_sync(gmask, valid ? o.code : -1, k, G);
+                if (code < 0) {  // past the end of the ray
                     done = true;
                     break;
                 }
-                const int code = __shfl_sync(gmask, o.code, k, G);
-                const float hfd = __shfl_sync(gmask, o.hfd, k, G);
-                const float E = __shfl_sync(gmask, o.E, k, G);
                 if (lane == 0) cnt.primary++;
                 if (MODE == kTraced && lane == 0) cnt.sig = (cnt.sig ^ (unsigned)code) * 16777619u;
-                if (code & kInCloud) apply(hfd, E);
+                if (code & kInCloud) {
+                    const float hfd = __shfl_sync(gmask, o.hfd, k, G);
+                    const float E = __shfl_sync(gmask, o.E, k, G);
+                    apply(hfd, E);
+                }
                 if (accum >= p.accum_limit) {
                     accum = 1.0f;
                     done = true;
