@@ -134,7 +134,7 @@ constexpr int kGodTaps = 100, kGodWarps = 4;
 // Rows a thread, by pixels: more share more of a tap, fewer leave more CTAs
 // (1 | 2 | 4 rows, us: 320x180 25 | 42 | -, 640x360 54 | 50 | -, 1280x720 141 | 127 | 140,
 // 1920x1080 283 | 239 | 237, 3840x2160 1044 | 839 | 785).
-constexpr long long kGodRows2 = 200000, kGodRows4 = 1800000;
+constexpr long long kRows2 = 200000, kRows4 = 1800000;
 
 // One axis' first tap, its step and whether all its taps keep a texel and a half
 // from the ends (the recurrence's roundings move a tap by less than a tenth of
@@ -274,19 +274,58 @@ MT_HD uint32_t unorm8(float f) {
     return (uint32_t)__float2uint_rn(c * 255.0f);
 }
 
-__global__ void __launch_bounds__(256) tonemap_kernel(TonemapArgs a) {
-    const int px = blockIdx.x * blockDim.x + threadIdx.x, py = blockIdx.y * blockDim.y + threadIdx.y;
-    if (px >= a.width || py >= a.height) return;
-    const int fx = winner_fragment(px, a.width), fy = winner_fragment(py, a.height);
-    if (fx < 0 || fy < 0) return;  // no fragment stores here: the pixel keeps its contents
-    const f4v c = tex2_border(a.in, a.width, a.height, frag_uv(fx, a.width), frag_uv(fy, a.height));
-    const float noise = wang_hash_noise((uint32_t)px, (uint32_t)py, f2u(a.time_y)) * 0.01f;
-    const float r = tonemap1(c.x) + noise, g = tonemap1(c.y) + noise, b = tonemap1(c.z) + noise;
-    const size_t idx = (size_t)py * (size_t)a.width + (size_t)px;
-    if (a.format == MT_LDR_RGBA8) {
-        static_cast<uint32_t*>(a.out)[idx] = unorm8(r) | (unorm8(g) << 8) | (unorm8(b) << 16) | (255u << 24);
-    } else {
-        static_cast<float4*>(a.out)[idx] = make_float4(r, g, b, 1.0f);
+// One axis of a pixel's filtered fetch: the fragment that stores to it (negative:
+// none) and where that fragment samples.
+struct ToneAxis {
+    int fragment, i;
+    float w;
+};
+MT_HD ToneAxis tone_axis(int p, int n) {
+    ToneAxis t;
+    t.fragment = winner_fragment(p, n);
+    const float u = frag_uv(t.fragment, n) * (float)n - 0.5f, fu = floorf(u);
+    t.i = f2i(fu);
+    t.w = u - fu;
+    return t;
+}
+
+// The tone map.  Bound by instruction issue (three powf and three divisions a
+// pixel), with 24 bytes a pixel far below it.  As in the blur, a pixel's column and
+// row are each looked up along one axis: a thread takes ROWS pixels of a column and
+// finds it once, a CTA's first threads find its rows once for the 32 columns.  The
+// blur's size lines hold here too (every pixel alone | 2 | 4 rows a thread, us:
+// 800x450 9 | 9 | 11, 1280x720 17 | 15 | 17, 1920x1080 34 | 29 | 29, 3840x2160
+// 122 | 101 | 97).
+constexpr int kToneWarps = 8;
+
+template <int ROWS, bool RGBA8>
+__global__ void __launch_bounds__(32 * kToneWarps) tonemap_kernel(const __grid_constant__ TonemapArgs a) {
+    constexpr int TH = kToneWarps * ROWS;
+    __shared__ ToneAxis rows[ROWS == 1 ? 1 : TH];
+    const int first = ((int)threadIdx.x >> 5) * ROWS;  // the thread's first row in the tile
+    const int px = (int)blockIdx.x * 32 + ((int)threadIdx.x & 31), y0 = (int)blockIdx.y * TH;
+    if (ROWS > 1) {
+        if (threadIdx.x < TH) rows[threadIdx.x] = tone_axis(y0 + (int)threadIdx.x, a.height);
+        __syncthreads();
+    }
+    if (px >= a.width) return;
+    const ToneAxis col = tone_axis(px, a.width);
+    if (col.fragment < 0) return;  // no fragment stores here: the pixel keeps its contents
+    const uint32_t time = f2u(a.time_y);
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+        const int py = y0 + first + k;
+        if (py >= a.height) return;
+        const ToneAxis row = ROWS == 1 ? tone_axis(py, a.height) : rows[first + k];
+        if (row.fragment < 0) continue;
+        const f4v c = tex2_border_at(a.in, a.width, a.height, col.i, col.w, row.i, row.w);
+        const float noise = wang_hash_noise((uint32_t)px, (uint32_t)py, time) * 0.01f;
+        const float r = tonemap1(c.x) + noise, g = tonemap1(c.y) + noise, b = tonemap1(c.z) + noise;
+        const size_t idx = (size_t)py * (size_t)a.width + (size_t)px;
+        if (RGBA8)
+            static_cast<uint32_t*>(a.out)[idx] = unorm8(r) | (unorm8(g) << 8) | (unorm8(b) << 16) | (255u << 24);
+        else
+            static_cast<float4*>(a.out)[idx] = make_float4(r, g, b, 1.0f);
     }
 }
 
@@ -295,18 +334,33 @@ __global__ void __launch_bounds__(256) tonemap_kernel(TonemapArgs a) {
 cudaError_t launch_godrays(const GodrayArgs& a, cudaStream_t s) {
     const unsigned gx = (unsigned)((a.width + 31) / 32);
     const long long pixels = (long long)a.width * a.height;
-    if (pixels >= kGodRows4)
+    if (pixels >= kRows4)
         godrays_kernel<4><<<dim3(gx, (unsigned)((a.height + 15) / 16)), 128, 0, s>>>(a);
-    else if (pixels >= kGodRows2)
+    else if (pixels >= kRows2)
         godrays_kernel<2><<<dim3(gx, (unsigned)((a.height + 7) / 8)), 128, 0, s>>>(a);
     else
         godrays_kernel<1><<<dim3(gx, (unsigned)((a.height + 3) / 4)), 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 
+namespace {
+template <int ROWS> void launch_tonemap_rows(const TonemapArgs& a, cudaStream_t s) {
+    const dim3 grid((unsigned)((a.width + 31) / 32), (unsigned)((a.height + kToneWarps * ROWS - 1) / (kToneWarps * ROWS)));
+    if (a.format == MT_LDR_RGBA8)
+        tonemap_kernel<ROWS, true><<<grid, 32 * kToneWarps, 0, s>>>(a);
+    else
+        tonemap_kernel<ROWS, false><<<grid, 32 * kToneWarps, 0, s>>>(a);
+}
+}  // namespace
+
 cudaError_t launch_tonemap(const TonemapArgs& a, cudaStream_t s) {
-    const dim3 block(32, 8), grid((a.width + 31) / 32, (a.height + 7) / 8);
-    tonemap_kernel<<<grid, block, 0, s>>>(a);
+    const long long pixels = (long long)a.width * a.height;
+    if (pixels >= kRows4)
+        launch_tonemap_rows<4>(a, s);
+    else if (pixels >= kRows2)
+        launch_tonemap_rows<2>(a, s);
+    else
+        launch_tonemap_rows<1>(a, s);
     return cudaGetLastError();
 }
 

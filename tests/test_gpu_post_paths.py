@@ -2,8 +2,9 @@
 import numpy as np
 import pytest
 
-from meteoros_gb300 import scenes
+from meteoros_gb300 import abi, scenes
 from tests.gpu_util import assert_bits_equal, to_dev
+from tests.test_gpu_post import check_tonemap
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +81,15 @@ def vctx(lib):
     c.generate_volumes(7)
     yield c
     c.close()
+
+
+# The tone map takes 1, 2 or 4 rows a thread by the image's size, their columns and
+# rows looked up apart: both sides of the size lines, images smaller than a tile.
+@pytest.mark.parametrize("size", [(1, 1), (3, 70), (33, 17), (448, 446), (447, 448), (1700, 1058), (1700, 1059)])
+def test_tonemap_forms_vs_oracle(ctx, oracle, size):
+    w, h = size
+    rng = np.random.default_rng(w * 31 + h)
+    img = rng.random((h, w, 4), dtype=np.float32) * np.float32(3.0)
+    tm = abi.time_init()
+    tm.time[1] = 2.5
+    check_tonemap(ctx, oracle, tm, img, f"{size}")
