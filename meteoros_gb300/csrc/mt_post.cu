@@ -8,12 +8,14 @@
 //
 // Both shaders run one fragment per pixel (in_uv at the pixel centre) and
 // store with imageStore at pixelPos = clamp(round(dim * in_uv)), which is the
-// fragment's own pixel or the next one.  One thread here owns one OUTPUT
-// pixel p and finds the fragment whose store lands there: along each axis the
-// candidates are fragments p and p - 1, and where both map to p the later one
-// in raster order (the larger index) wins.  Each output pixel is written by
-// exactly one thread, so the result is defined (in the reference, colliding
-// stores race) and out may alias in.
+// fragment's own pixel or the next one.  The fragment whose store lands on a
+// pixel p: along each axis the candidates are fragments p and p - 1, and where
+// both map to p the later one in raster order (the larger index) wins.  The tone
+// map's threads own pixels and find their fragments; the blur's own fragments and
+// write the pixels they win, and a pixel that no fragment stores to is copied by
+// the thread of its own index.  Each output pixel is read and written by exactly
+// one thread, so the result is defined (in the reference, colliding stores race),
+// and the blur's out may alias in.
 //
 // Compiled with -fmad=false and IEEE division: the operation order follows
 // the shaders' so the results equal the CPU restatement bit for bit except
@@ -117,69 +119,123 @@ MT_HD GodrayFrame godray_frame(const mt_camera_ubo& cam) {
     return g;
 }
 
-// The blur.  Bound by instruction issue: 100 bilinear taps a pixel, each with its
-// coordinates, four loads, nine interpolation operations and the channels'
-// weighted sums.  A pixel's taps step along a line, ux -= dx and uy -= dy on every
-// tap, so their columns depend on the pixel's column alone and their rows on its
-// row.  A thread takes ROWS pixels of one column and computes each tap's column
-// once for all of them; a CTA's first threads tabulate the taps' rows in shared
-// memory, a thread a row of pixels (small images, where that table's serial chain
-// would be the time: one pixel a thread, its rows its own).  A CTA whose taps all
-// lie inside the image (coordinates move monotonically, so the ends decide)
-// takes the loop without border checks, and one sum serves red and green where
-// the light's are equal, as the reference's are.
+// The blur.  Bound by instruction issue and texel latency: 100 bilinear taps a
+// fragment, each with its coordinates, loads, nine interpolation operations and the
+// channels' weighted sums.  A fragment's taps step along a line, ux -= dx and
+// uy -= dy on every tap, so their columns depend on its column alone and their rows
+// on its row.  A thread takes ROWS fragments of one column and computes each tap's
+// column once for all of them; a CTA's first threads step through the taps' rows,
+// whose texels and weights all of them then tabulate in shared memory (small images,
+// where the steps' serial chain would be the time: one fragment a thread, its rows
+// its own).  A CTA whose taps all lie inside the image (coordinates move
+// monotonically, so the ends decide) takes the loop without border checks, where
+// neighbouring rows share filtered texels (god_blur), and one sum serves red and
+// green where the light's are equal, as the reference's are.
 // One pixel a thread with its own taps and border checks took 409 us at 1080p and
-// 1.58 ms at 4K (430 M warp instructions at 1080p); now 237 us and 0.79 ms (173 M).
+// 1.58 ms at 4K (430 M warp instructions at 1080p); rows and columns looked up apart
+// 237 us and 0.79 ms (173 M); threads over fragments, whose rows are one apart where
+// pixels' fragments repeat and skip, sharing filtered texels 222 us and 0.71 ms
+// (unrolled by 2, 224 us).
 constexpr int kGodTaps = 100, kGodWarps = 4;
 // Rows a thread, by pixels: more share more of a tap, fewer leave more CTAs
-// (1 | 2 | 4 rows, us: 320x180 25 | 42 | -, 640x360 54 | 50 | -, 1280x720 141 | 127 | 140,
-// 1920x1080 283 | 239 | 237, 3840x2160 1044 | 839 | 785).
+// (1 | 2 | 4 rows, us: 320x180 25 | 42 | -, 640x360 54 | 44 | -, 1280x720 141 | 121 | -,
+// 1920x1080 283 | 229 | 222; 8 rows 268).
 constexpr long long kRows2 = 200000, kRows4 = 1800000;
 
-// One axis' first tap, its step and whether all its taps keep a texel and a half
-// from the ends (the recurrence's roundings move a tap by less than a tenth of
-// one).  A pixel that no fragment stores to is blurred from a fragment of its
-// own and keeps its input.
+// One axis of a fragment: its first tap, its step and whether all its taps keep a
+// texel and a half from the ends (the recurrence's roundings move a tap by less
+// than a tenth of one); the pixel it stores to (negative: a later fragment stores
+// there too); and whether any fragment stores to the pixel of its own index, which
+// keeps its input otherwise.
 struct GodAxis {
     float u, d;
-    int fragment;
-    bool inside;
+    int pixel;
+    bool covered, inside;
 };
-MT_HD GodAxis god_axis(int p, int n, float ss) {
+MT_HD GodAxis god_axis(int f, int n, float ss) {
     GodAxis x;
-    p = imin(p, n - 1);
-    x.fragment = winner_fragment(p, n);
-    x.u = frag_uv(x.fragment >= 0 ? x.fragment : p, n);
+    f = imin(f, n - 1);
+    const int p = frag_pixel(f, n);
+    x.pixel = winner_fragment(p, n) == f ? p : -1;
+    x.covered = winner_fragment(f, n) >= 0;
+    x.u = frag_uv(f, n);
     x.d = ((x.u - ss) / 100.0f) * 1.0f;
     const float lo = 1.5f / (float)n, hi = 1.0f - 2.5f / (float)n, last = x.u + (ss - x.u) * 0.99f;
     x.inside = x.u >= lo && x.u <= hi && last >= lo && last <= hi;
     return x;
 }
 
-// The sums of a thread's pixels, ROWS rows of one column from the table's row on.
+// The sums of a thread's fragments, ROWS rows of one column from the table's row on.
+// INSIDE: no tap touches the border; and, for several rows, from the second tap on
+// each row taps the texel row of the row above it or the next, as fragments
+// close in on the sun together.  Then the rows' filtered texels chain: a row's
+// upper texels are its upper neighbour's, upper or lower, and it loads and filters
+// its lower two, in packed pairs of rows.
 template <int ROWS, bool INSIDE, bool SHARED_RG>
-MT_HD void god_blur(const GodrayArgs& a, const AxisTap* rows, GodAxis col, GodAxis row, float (&ax)[ROWS],
-                    float (&ay)[ROWS], float (&az)[ROWS]) {
+MT_HD void god_blur(const GodrayArgs& a, const AxisTap* rows, GodAxis col, GodAxis row, float2 (&ax)[(ROWS + 1) / 2],
+                    float2 (&ay)[(ROWS + 1) / 2], float2 (&az)[(ROWS + 1) / 2]) {
+    constexpr int TH = kGodWarps * ROWS, PAIRS = (ROWS + 1) / 2;
     const float w = 1.0f * 0.001f;  // illuminationDecay * WEIGHT_FOR_SAMPLE, DECAY = 1
     const float fw = (float)a.width, fh = (float)a.height;
-    constexpr int kUnroll = ROWS == 1 ? 4 : 2;
-#pragma unroll kUnroll
-    for (int i = 0; i < kGodTaps; ++i) {
+    auto add = [&](int k, float2 s) {
+        auto weighted = [&](float light) { return mul2(mul2(splat2(light), s), splat2(w)); };
+        ax[k] = add2(ax[k], weighted(a.light[0]));
+        if (!SHARED_RG) ay[k] = add2(ay[k], weighted(a.light[1]));
+        az[k] = add2(az[k], weighted(a.light[2]));
+    };
+    auto single = [&](int i) {
         const AxisTap x = axis_tap(col.u, fw);
 #pragma unroll
-        for (int k = 0; k < ROWS; ++k) {
-            const AxisTap y = ROWS == 1 ? axis_tap(row.u, fh) : rows[i * (kGodWarps * ROWS) + k];
-            const float s = mask_decode<INSIDE>(a, x, y);
-            ax[k] += (a.light[0] * s) * w;
-            if (!SHARED_RG) ay[k] += (a.light[1] * s) * w;
-            az[k] += (a.light[2] * s) * w;
+        for (int k = 0; k < PAIRS; ++k) {
+            float s[2] = {0.0f, 0.0f};
+#pragma unroll
+            for (int h = 0; h < 2 && 2 * k + h < ROWS; ++h) {
+                const AxisTap y = ROWS == 1 ? axis_tap(row.u, fh) : rows[i * TH + 2 * k + h];
+                s[h] = mask_decode<INSIDE>(a, x, y);
+            }
+            add(k, make_float2(s[0], s[1]));
         }
         col.u -= col.d;
         if (ROWS == 1) row.u -= row.d;
+    };
+    if (INSIDE && ROWS > 1) {
+        single(0);
+#pragma unroll 1
+        for (int i = 1; i < kGodTaps; ++i) {
+            const AxisTap x = axis_tap(col.u, fw);
+            const int lower = x.i + a.width;
+            int last = 0;
+            float up = 0.0f, down = 0.0f;  // the last row's filtered texels
+#pragma unroll
+            for (int k = 0; k < PAIRS; ++k) {
+                const float4 t = *reinterpret_cast<const float4*>(rows + i * TH + 2 * k);
+                const int j0 = __float_as_int(t.y), j1 = __float_as_int(t.w);
+                const float *r0 = a.mask + (j0 * a.width + lower), *r1 = a.mask + (j1 * a.width + lower);
+                const float2 d = lerp2(make_float2(__ldg(r0), __ldg(r1)), make_float2(__ldg(r0 + 1), __ldg(r1 + 1)),
+                                       splat2(x.w));
+                float2 u;
+                if (k == 0) {
+                    const float* r = a.mask + (j0 * a.width + x.i);
+                    u.x = lerp1(__ldg(r), __ldg(r + 1), x.w);
+                } else {
+                    u.x = j0 != last ? down : up;
+                }
+                u.y = j1 != j0 ? d.x : u.x;
+                add(k, lerp2(u, d, make_float2(t.x, t.z)));
+                last = j1;
+                up = u.y;
+                down = d.y;
+            }
+            col.u -= col.d;
+        }
+    } else {
+        constexpr int kUnroll = ROWS == 1 ? 4 : 2;
+#pragma unroll kUnroll
+        for (int i = 0; i < kGodTaps; ++i) single(i);
     }
     if (SHARED_RG) {
 #pragma unroll
-        for (int k = 0; k < ROWS; ++k) ay[k] = ax[k];
+        for (int k = 0; k < PAIRS; ++k) ay[k] = ax[k];
     }
 }
 
@@ -188,7 +244,8 @@ __global__ void __launch_bounds__(32 * kGodWarps) godrays_kernel(const __grid_co
     constexpr int TH = kGodWarps * ROWS;
     __shared__ __align__(16) AxisTap taps[ROWS == 1 ? 1 : kGodTaps * TH];
     __shared__ GodrayFrame frame;
-    __shared__ int fragment_y[TH];
+    __shared__ int pixel_y[TH];
+    __shared__ bool covered_y[TH];
     const int W = a.width, H = a.height;
     const int first = ((int)threadIdx.x >> 5) * ROWS;  // the thread's first row in the tile
     const int px = (int)blockIdx.x * 32 + ((int)threadIdx.x & 31), y0 = (int)blockIdx.y * TH;
@@ -203,18 +260,29 @@ __global__ void __launch_bounds__(32 * kGodWarps) godrays_kernel(const __grid_co
     bool inside = col.inside && row.inside;
     inside = ROWS == 1 ? __all_sync(0xffffffffu, inside) != 0 : __syncthreads_and(inside) != 0;
     if (ROWS > 1) {
+        bool chain = true;
         if (threadIdx.x < TH) {
-            fragment_y[threadIdx.x] = row.fragment;
+            pixel_y[threadIdx.x] = row.pixel;
+            covered_y[threadIdx.x] = row.covered;
+#pragma unroll 10
             for (int i = 0; i < kGodTaps; ++i) {
-                taps[i * TH + threadIdx.x] = axis_tap(row.u, (float)H);
+                taps[i * TH + threadIdx.x].w = row.u;
                 row.u -= row.d;
             }
         }
         __syncthreads();
+        for (int e = (int)threadIdx.x; e < kGodTaps * TH; e += 32 * kGodWarps) {  // whole warps
+            const AxisTap y = axis_tap(taps[e].w, (float)H);
+            const int below = __shfl_down_sync(0xffffffffu, y.i, 1, TH);
+            chain = chain && (e < TH || (unsigned)below - (unsigned)y.i <= 1u);
+            taps[e] = y;
+        }
+        inside = __syncthreads_and(chain) != 0 && inside;
     }
-    float ax[ROWS], ay[ROWS], az[ROWS];
+    constexpr int PAIRS = (ROWS + 1) / 2;
+    float2 ax[PAIRS], ay[PAIRS], az[PAIRS];
 #pragma unroll
-    for (int k = 0; k < ROWS; ++k) ax[k] = ay[k] = az[k] = 0.0f;
+    for (int k = 0; k < PAIRS; ++k) ax[k] = ay[k] = az[k] = make_float2(0.0f, 0.0f);
     if (!(g.blend < 0.0f) && !g.outside) {
         if (inside && a.light[0] == a.light[1])
             god_blur<ROWS, true, true>(a, taps + first, col, row, ax, ay, az);
@@ -228,13 +296,20 @@ __global__ void __launch_bounds__(32 * kGodWarps) godrays_kernel(const __grid_co
     for (int k = 0; k < ROWS; ++k) {
         const int py = y0 + first + k;
         if (py >= H) return;
-        const size_t idx = (size_t)py * (size_t)W + (size_t)px;
+        if (!(col.covered && (ROWS == 1 ? row.covered : covered_y[first + k]))) {  // the pixel of this index
+            const size_t own = (size_t)py * (size_t)W + (size_t)px;
+            a.out[own] = a.in[own];
+        }
+        const int y = ROWS == 1 ? row.pixel : pixel_y[first + k];
+        if (col.pixel < 0 || y < 0) continue;
+        const size_t idx = (size_t)y * (size_t)W + (size_t)col.pixel;
         float4 v = a.in[idx];
-        if (col.fragment >= 0 && (ROWS == 1 ? row.fragment : fragment_y[first + k]) >= 0 && !(g.blend < 0.0f)) {
+        if (!(g.blend < 0.0f)) {
             // the out-of-frustum branch discards what it accumulated (:126)
-            v.x += (ax[k] * 1.0f) * g.blend;
-            v.y += (ay[k] * 1.0f) * g.blend;
-            v.z += (az[k] * 1.0f) * g.blend;
+            auto of = [&](const float2(&sums)[PAIRS]) { return k & 1 ? sums[k / 2].y : sums[k / 2].x; };
+            v.x += (of(ax) * 1.0f) * g.blend;
+            v.y += (of(ay) * 1.0f) * g.blend;
+            v.z += (of(az) * 1.0f) * g.blend;
             v.w += 1.0f * g.blend;
         }
         a.out[idx] = v;

@@ -13,13 +13,13 @@ cases:
   batch_fp16      the same with FP16 volumes
   precision       3840x2160 full frame, FP16 volumes (march_kernel<1>, half2 path)
   precision_bf16  the same frame with bfloat16 volumes (filtered in FP32)
-  upload          host RGBA8 volumes uploaded: the 16-bit copies (u8_to_16_kernel) and the
-                  samplers' layouts (quads3_kernel, quads16_kernel, cells2_kernel)
+  upload          host RGBA8 volumes uploaded: the 16-bit copies and the samplers' layouts
+                  (layouts_kernel)
   batch_noalloc   16 views through the allocation-free batch entry (noalloc_store_kernel,
                   noalloc_tiles_kernel, march_batch_kernel)
   godrays         1920x1080 god-ray radial blur
   tonemap         1920x1080 tone map + dither to RGBA8
-  generate        noise-volume generation (gen_* kernels)
+  generate        noise-volume generation (gen_volumes_kernel, layouts_kernel)
   frame_fused     the 1080p reprojected frame with the reprojection fused into the TXAA
                   resolve (resolve_kernel)
   tga             a 128-slice stack of 128x128 run-length TGA files decoded on the device

@@ -37,6 +37,9 @@ def test_godray_forms_bit_exact(ctx, oracle, size, light):
         ctx.godrays(cam, light, to_dev(mask, torch), to_dev(img, torch), out)
         want = oracle.godrays(cam, np.array(light, np.float32), mask, img)
         assert_bits_equal(out.cpu().numpy(), want, f"{size} yaw {yaw}")
+        same = to_dev(img, torch)  # in place
+        ctx.godrays(cam, light, to_dev(mask, torch), same, same)
+        assert_bits_equal(same.cpu().numpy(), want, f"{size} yaw {yaw} in place")
 
 
 # The previous camera's uv checks three denominators instead of eleven quotients
