@@ -222,7 +222,7 @@ struct ForkJoin {
 
 cudaError_t launch_render(const MarchArgs& a, cudaStream_t s, const LaunchEvents* ev, const ForkJoin* fj);
 cudaError_t launch_reproject(const MarchArgs& a, cudaStream_t s);
-cudaError_t launch_march_u8(const MarchArgs& a, cudaStream_t s, long long rays);
+cudaError_t launch_march_u8(const MarchArgs& a, cudaStream_t s);
 // Persistent batched march: `blocks` CTAs of 128 threads, `lanes` per ray.
 cudaError_t launch_batch_u8(const BatchArgs& b, int lanes, int blocks, cudaStream_t s);
 cudaError_t launch_batch_f16(const BatchArgs& b, int lanes, int blocks, cudaStream_t s);
@@ -231,8 +231,8 @@ cudaError_t launch_batch_bf16(const BatchArgs& b, int lanes, int blocks, cudaStr
 int batch_blocks_u8(int device, int lanes);
 int batch_blocks_f16(int device, int lanes);
 int batch_blocks_bf16(int device, int lanes);
-cudaError_t launch_march_f16(const MarchArgs& a, cudaStream_t s, long long rays);
-cudaError_t launch_march_bf16(const MarchArgs& a, cudaStream_t s, long long rays);
+cudaError_t launch_march_f16(const MarchArgs& a, cudaStream_t s);
+cudaError_t launch_march_bf16(const MarchArgs& a, cudaStream_t s);
 cudaError_t launch_txaa(const TxaaArgs& a, cudaStream_t s, const cudaEvent_t* ev);
 cudaError_t launch_godrays(const GodrayArgs& a, cudaStream_t s);
 // Slices of 2^log2n x 2^log2n pixels.

@@ -492,7 +492,9 @@ MT_HD void march_pixel(const MarchArgs& a, const Frame& F, const Tex<S>& tx, int
 // groups_x x groups_y blocks of 4x4 (Renderer.cpp:713-716); each ray is one
 // block's slot pixel.  Full: one ray per pixel.  G consecutive lanes (an
 // aligned segment of a warp) march one ray.  BS threads per CTA (256 by
-// default, 128 or 32 selectable).  Resident threads per SM: 1024 (64 registers
+// default, 128 or 32 selectable; 128 at most for one and two lanes per ray, whose
+// rays end furthest apart: 960x540 full frames 357 / 234 -> 344 / 230 us by view, FP16
+// 4K 3.76 / 2.58 -> 3.70 / 2.54 ms, 640x360 full frame 205 / 140 -> 196 / 139).  Resident threads per SM: 1024 (64 registers
 // a thread), or for one lane per ray on FP16 volumes 1280 (48, with some 200 B
 // of spills: 4K 4.12 ms for 4.19; RGBA8 took 4.69 ms so for 4.62, and bfloat16
 // 1603x901 1.06 ms for 1.01).
@@ -504,6 +506,20 @@ constexpr int march_min_blocks(int G, int S, int BS) {
     const int n = (G == 1 && S == MT_STORAGE_F16 ? 1280 : 1024) / BS;
     return n < 32 ? n : 32;  // at most 32 CTAs an SM
 }
+// The rays of a warp.  One lane per ray: 8x4 rays, which fetch nearer cells and end
+// nearer one another than 32 in a row (960x540 full frames 387 / 235 -> 357 / 234 us by
+// view, bfloat16 1603x901 976 / 604 -> 892 / 589, 3840x2160 frame 628 / 523 ->
+// 607 / 518).  More lanes: a row of rays (2 lanes on 4x4 rays: 640x360 full frame
+// 196 / 139 -> 190 / 138, but 2560x1440 frame 307 / 267 -> 304 / 277).
+template <int G> struct WarpTile {
+    static constexpr int R = 32 / G, W = R >= 32 ? 8 : R, H = R / W;
+    // the launch's rays in whole tiles
+    static long long rays(const MarchArgs& a) {
+        const bool full = (a.flags & MT_RENDER_FULL) != 0;
+        const long long nx = full ? a.width : a.groups_x, ny = full ? a.height : a.groups_y;
+        return (nx + W - 1) / W * ((ny + H - 1) / H) * R;
+    }
+};
 template <int G, int S, int BS, int MODE>
 __global__ void __launch_bounds__(BS, march_min_blocks(G, S, BS))
     march_kernel(const __grid_constant__ MarchArgs a) {
@@ -521,20 +537,22 @@ __global__ void __launch_bounds__(BS, march_min_blocks(G, S, BS))
     unsigned pixels = 0;
     int px = 0, py = 0;
     bool active;
-    if (a.flags & MT_RENDER_FULL) {
-        active = (long long)idx < (long long)a.width * a.height;
-        if (active) {
-            px = (int)(idx % (unsigned)a.width);
-            py = march_row((int)(idx / (unsigned)a.width), a.height, a.bottom_up);
-        }
+    using T = WarpTile<G>;
+    const bool full = (a.flags & MT_RENDER_FULL) != 0;
+    const int nx = full ? a.width : a.groups_x, ny = full ? a.height : a.groups_y;
+    const unsigned cols = (unsigned)(nx + T::W - 1) / T::W, rows = (unsigned)(ny + T::H - 1) / T::H;
+    const unsigned tile = idx / T::R, sub = idx % T::R;
+    const int rx = (int)(tile % cols * T::W + sub % T::W);
+    const int ry = march_row((int)(tile / cols), (int)rows, a.bottom_up) * T::H + (int)(sub / T::W);
+    active = tile / cols < rows && rx < nx && ry < ny;
+    if (full) {
+        px = rx;
+        py = ry;
     } else {
-        active = (long long)idx < (long long)a.groups_x * a.groups_y;
-        if (active) {
-            const int id = a.time.frame_count_mod16;
-            px = (int)(idx % (unsigned)a.groups_x) * 4 + a.params.slot_x[id];
-            py = march_row((int)(idx / (unsigned)a.groups_x), a.groups_y, a.bottom_up) * 4 + a.params.slot_y[id];
-            active = px < a.width && py < a.height;
-        }
+        const int id = a.time.frame_count_mod16;
+        px = rx * 4 + a.params.slot_x[id];
+        py = ry * 4 + a.params.slot_y[id];
+        active = active && px < a.width && py < a.height;
     }
     if (active) {
         march_pixel<G, S, MODE>(a, F, tx, px, py, cnt, gmask, lane, s_jitter);
@@ -617,42 +635,42 @@ template <int S> int batch_blocks_storage(int device, int lanes) {
     return (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
 }
 
-template <int S, int BS> void launch_march_bs(const MarchArgs& a, cudaStream_t s, long long rays) {
-    const int G = a.lanes;
-    const unsigned blocks = (unsigned)((rays * G + BS - 1) / BS);
-    switch (G) {
-        case 1: march_kernel<1, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
-        case 2: march_kernel<2, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
-        case 32: march_kernel<32, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
-        case 4: march_kernel<4, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
-        case 16: march_kernel<16, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
-        default: march_kernel<8, S, BS, kTame><<<blocks, BS, 0, s>>>(a); break;
+template <int G, int S, int BS, int MODE> void launch_march_kernel(const MarchArgs& a, cudaStream_t s) {
+    const unsigned blocks = (unsigned)((WarpTile<G>::rays(a) * G + BS - 1) / BS);
+    march_kernel<G, S, BS, MODE><<<blocks, BS, 0, s>>>(a);
+}
+
+// The CTA size asked for, 128 threads at most for one and two lanes per ray.
+template <int S, int BS> void launch_march_bs(const MarchArgs& a, cudaStream_t s) {
+    constexpr int BS2 = BS < 128 ? BS : 128;
+    switch (a.lanes) {
+        case 1: launch_march_kernel<1, S, BS2, kTame>(a, s); break;
+        case 2: launch_march_kernel<2, S, BS2, kTame>(a, s); break;
+        case 4: launch_march_kernel<4, S, BS, kTame>(a, s); break;
+        case 16: launch_march_kernel<16, S, BS, kTame>(a, s); break;
+        case 32: launch_march_kernel<32, S, BS, kTame>(a, s); break;
+        default: launch_march_kernel<8, S, BS, kTame>(a, s); break;
     }
 }
 
-template <int S> cudaError_t launch_march_storage(const MarchArgs& a, cudaStream_t s, long long rays) {
-    if (a.trace || !a.frame.tame) {  // 256-thread CTAs, 1 or 4 lanes
-        const int G = a.lanes == 1 ? 1 : 4;
-        const unsigned blocks = (unsigned)((rays * G + 255) / 256);
-        if (a.trace) {
-            if (G == 1)
-                march_kernel<1, S, 256, kTraced><<<blocks, 256, 0, s>>>(a);
-            else
-                march_kernel<4, S, 256, kTraced><<<blocks, 256, 0, s>>>(a);
-        } else {
-            if (G == 1)
-                march_kernel<1, S, 256, kGeneral><<<blocks, 256, 0, s>>>(a);
-            else
-                march_kernel<4, S, 256, kGeneral><<<blocks, 256, 0, s>>>(a);
-        }
-        return cudaGetLastError();
+template <int S> cudaError_t launch_march_storage(const MarchArgs& a, cudaStream_t s) {
+    if (a.trace) {  // 256-thread CTAs, 1 or 4 lanes
+        if (a.lanes == 1)
+            launch_march_kernel<1, S, 256, kTraced>(a, s);
+        else
+            launch_march_kernel<4, S, 256, kTraced>(a, s);
+    } else if (!a.frame.tame) {
+        if (a.lanes == 1)
+            launch_march_kernel<1, S, 256, kGeneral>(a, s);
+        else
+            launch_march_kernel<4, S, 256, kGeneral>(a, s);
+    } else if (a.block == 256) {
+        launch_march_bs<S, 256>(a, s);
+    } else if (a.block == 128) {
+        launch_march_bs<S, 128>(a, s);
+    } else {
+        launch_march_bs<S, 32>(a, s);
     }
-    if (a.block == 256)
-        launch_march_bs<S, 256>(a, s, rays);
-    else if (a.block == 128)
-        launch_march_bs<S, 128>(a, s, rays);
-    else
-        launch_march_bs<S, 32>(a, s, rays);
     return cudaGetLastError();
 }
 

@@ -2,8 +2,8 @@
 #include "mt_march.cuh"
 
 namespace mt {
-cudaError_t launch_march_f16(const MarchArgs& a, cudaStream_t s, long long rays) {
-    return launch_march_storage<MT_STORAGE_F16>(a, s, rays);
+cudaError_t launch_march_f16(const MarchArgs& a, cudaStream_t s) {
+    return launch_march_storage<MT_STORAGE_F16>(a, s);
 }
 cudaError_t launch_batch_f16(const BatchArgs& b, int lanes, int blocks, cudaStream_t s) {
     return launch_batch_storage<MT_STORAGE_F16>(b, lanes, blocks, s);

@@ -416,9 +416,9 @@ static cudaError_t launch_march(const MarchArgs& a, cudaStream_t s, const Launch
     cudaError_t e = cudaSuccess;
     if (m > 0) {
         switch (a.params.storage) {
-            case MT_STORAGE_F16: e = launch_march_f16(a, s, m); break;
-            case MT_STORAGE_BF16: e = launch_march_bf16(a, s, m); break;
-            default: e = launch_march_u8(a, s, m); break;
+            case MT_STORAGE_F16: e = launch_march_f16(a, s); break;
+            case MT_STORAGE_BF16: e = launch_march_bf16(a, s); break;
+            default: e = launch_march_u8(a, s); break;
         }
     }
     if (timed) cudaEventRecord(ev->march[1], s);

@@ -161,3 +161,23 @@ def test_coverage_bounds_equal_oracle(ctx, oracle, vol7, coverage):
     cam, tm, params, _ = scenes.config_view(3, W, H)
     params.coverage_mode, params.coverage, params.height_gradient = 0, coverage, 1
     check_density(oracle, vol7, ctx, params, cam, tm)
+
+
+@pytest.mark.parametrize("size", [(1, 1), (7, 3), (8, 4), (9, 5), (65, 37), (130, 18)])
+def test_warp_tiles_march_every_ray_once(ctx, oracle, vol7, size):
+    """One-lane warps take 8x4 rays: grids smaller than a tile, whole tiles and one
+    ray more, either row order, every CTA size, full and checkerboard, against the
+    oracle's god-ray values and counters."""
+    w, h = size
+    cam, tm, params, _ = scenes.config_view(5, w, h)
+    prev = np.random.default_rng(w).random((h, w, 4), dtype=np.float32)
+    for flags in (abi.MT_RENDER_FULL, 0):
+        _, want, cnt = oracle.render(vol7, cam, cam, tm, params, prev, w, h, flags)
+        for order, block in ((0, 0), (1, 128), (0, 32)):
+            ctx.set_tuning(march_lanes=1, march_order=order, march_block=block)
+            try:
+                _, got, st = gpu_render(ctx, cam, cam, tm, params, prev, w, h, flags)
+            finally:
+                ctx.set_tuning(march_lanes=0, march_order=0, march_block=0)
+            assert_bits_equal(got, want, f"{size} flags {flags} order {order} block {block}")
+            assert (st.primary_samples, st.light_samples, st.marched_rays) == tuple(int(c) for c in cnt[:3])
