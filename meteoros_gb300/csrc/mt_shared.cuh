@@ -202,7 +202,7 @@ MT_HD float henyey_greenstein(float c, float e) {
 // only, never the accumulated density, the control flow or the god-ray mask.
 template <bool TAME, bool EXACT>
 MT_HD float light_energy(float h, float dl, float ds, float phase, float cos_q, float brightness) {
-    if (EXACT) {  // the same operations, special-function forms and clamps as single instructions
+    if (EXACT) {  // the same operations, clamps as single instructions
         const float primary = exp_ftz(-dl);
         const float att = fmaxf(primary + (cos_q * (primary * 0.25f - primary)), primary);
         const float e = fminf(fmaxf(remap_r<true>(h * 0.125f, 0.3f, MT_RCP(0.3f, 0.85f), 0.5f, 2.0f), 0.5f), 2.0f);
@@ -210,11 +210,11 @@ MT_HD float light_energy(float h, float dl, float ds, float phase, float cos_q, 
         const float in_scatter = (0.05f + pow_ftz(ds, e)) * pow_ftz(v, 0.8f);
         return att * primary * in_scatter * phase * brightness;
     }
-    const float primary = __expf(-dl);
+    const float primary = exp_ftz(-dl);
     const float secondary = primary;  // exp(-dl) twice in the reference (:334, :340)
     float att = gmax(secondary + (cos_q * (secondary * 0.25f - secondary)), primary);
-    float depth = 0.05f + __powf(ds, gclamp(remap_r<TAME>(h * 0.125f, 0.3f, MT_RCP(0.3f, 0.85f), 0.5f, 2.0f), 0.5f, 2.0f));
-    float vert = __powf(gclamp(remap_r<TAME>(h * 1.5f, 0.07f, MT_RCP(0.07f, 0.34f), 0.1f, 1.0f), 0.1f, 1.0f), 0.8f);
+    float depth = 0.05f + pow_ftz(ds, gclamp(remap_r<TAME>(h * 0.125f, 0.3f, MT_RCP(0.3f, 0.85f), 0.5f, 2.0f), 0.5f, 2.0f));
+    float vert = pow_ftz(gclamp(remap_r<TAME>(h * 1.5f, 0.07f, MT_RCP(0.07f, 0.34f), 0.1f, 1.0f), 0.1f, 1.0f), 0.8f);
     float in_scatter = depth * vert;
     return att * primary * in_scatter * phase * brightness;
 }
