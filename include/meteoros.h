@@ -303,7 +303,9 @@ MT_API mt_status mt_txaa(mt_ctx* ctx, const mt_camera_ubo* camera, const mt_came
  * host array; its image pointers are device pointers.  All views share one
  * storage.  Checkerboard views are reprojected first, then one persistent
  * raymarch launch takes tiles of every view from a work counter; the whole
- * batch is a CUDA graph launched on `stream`.  Results equal mt_render per view.
+ * batch is a CUDA graph launched on `stream`.  Results equal mt_render per view,
+ * also where a view's cur_rgba is an earlier view's prev_rgba: views that share
+ * an image are reprojected in view order.
  * Two batches may be in flight at once (on two streams they overlap on the
  * device); a third waits for the first.  The views' images of batches in
  * flight together must not overlap. */

@@ -19,6 +19,7 @@
 
 #include <cuda_runtime.h>
 
+#include "mt_batch.h"
 #include "mt_kernels.h"
 
 static_assert(MT_BASE_N == 1 << 7 && MT_DETAIL_N == 1 << 5, "the TGA decode's slice sizes");
@@ -791,6 +792,20 @@ void batch_shape(const mt_ctx* ctx, long long rays, int* lanes, int* tw, int* th
     }
 }
 
+// The graph branches a batch's reprojections may spread over: one, in view order,
+// where a view's frame is another's previous frame or the same image (a recycled
+// image is read before it is written, as when the views are rendered one by one).
+int reprojection_branches(const std::vector<mt::MarchArgs>& views) {
+    std::vector<mt::ImageBytes> images;
+    for (const mt::MarchArgs& a : views) {
+        if (a.flags & MT_RENDER_FULL) continue;
+        const size_t bytes = (size_t)a.width * (size_t)a.height * sizeof(float4);
+        images.push_back(mt::image_bytes(a.prev, bytes, false));
+        images.push_back(mt::image_bytes(a.cur, bytes, true));
+    }
+    return mt::written_overlap(std::move(images)) ? 1 : mt::kBatchBranches;
+}
+
 // The ray grid of a view: pixels (full) or the 4x4 blocks whose slot pixel
 // lies in the image and in the reference's dispatch (checkerboard).
 void ray_grid(const mt::MarchArgs& a, int* nrx, int* nry) {
@@ -911,6 +926,7 @@ MT_API mt_status mt_render_batch(mt_ctx* ctx, const mt_view* views, int n_views,
     // (one chain of them left the GPU idle between small views' launches: 24
     // sessions' frames 1.69 / 1.46 -> 1.63 / 1.41 ms; 2 branches 1.64 / 1.41, 8 the same
     // as 4), then the raymarch.
+    const int branches = reprojection_branches(args);
     cudaError_t e = cudaEventRecord(ctx->cap_fork, cs);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(ctx->d_views[k], h_views, args.size() * sizeof(mt::MarchArgs), cudaMemcpyHostToDevice, cs);
@@ -921,12 +937,12 @@ MT_API mt_status mt_render_batch(mt_ctx* ctx, const mt_view* views, int n_views,
     int reprojected = 0;
     for (int i = 0; e == cudaSuccess && i < n_views; ++i) {
         if (args[(size_t)i].flags & MT_RENDER_FULL) continue;
-        cudaStream_t branch = ctx->cap_branch[reprojected % mt::kBatchBranches];
-        if (reprojected++ < mt::kBatchBranches) e = cudaStreamWaitEvent(branch, ctx->cap_fork, 0);
+        cudaStream_t branch = ctx->cap_branch[reprojected % branches];
+        if (reprojected++ < branches) e = cudaStreamWaitEvent(branch, ctx->cap_fork, 0);
         if (e == cudaSuccess) e = mt::launch_reproject(args[(size_t)i], branch);
     }
     // joined whatever failed: the capture ends with every branch back on cs
-    for (int i = 0; i < std::min(reprojected, mt::kBatchBranches); ++i) {
+    for (int i = 0; i < std::min(reprojected, branches); ++i) {
         cudaError_t ej = cudaEventRecord(ctx->cap_join[i], ctx->cap_branch[i]);
         if (ej == cudaSuccess) ej = cudaStreamWaitEvent(cs, ctx->cap_join[i], 0);
         if (e == cudaSuccess) e = ej;
