@@ -337,7 +337,10 @@ MT_HD f3 ray_march_group(const mt_params& p, const Frame& F, const Tex<S>& tx, c
     const int shift = (int)(threadIdx.x & 31u) & ~(G - 1);  // the group's first lane
     float t_base = start_t;
     int s_base = 0;
-    bool done = false;
+    // A ray that ends before it begins (the two are distances from the origin, so a
+    // ray toward it from far away does) marches no step.  Without this its negative
+    // steps would bring later lanes of a long chunk below the end.
+    bool done = G > 4 && !(start_t < end_t);
     while (!done) {
         float t = t_base;
         for (int k = 0; k < lane; ++k) t += stepSize;
@@ -395,7 +398,7 @@ MT_HD f3 ray_march_group(const mt_params& p, const Frame& F, const Tex<S>& tx, c
             // limit not lie above 0): a loop over those, where the steps of a
             // long chunk one by one take four shuffles each.
             static_assert(G <= 4 || MODE != kTraced, "traced marches use 1 or 4 lanes");
-            const unsigned in_chunk = __ballot_sync(gmask, valid) >> shift & kGroup;  // the first steps
+            const unsigned in_chunk = __ballot_sync(gmask, valid) >> shift & kGroup;  // the first steps: t grows
             const unsigned cloud = __ballot_sync(gmask, (o.code & kInCloud) != 0) >> shift & kGroup;
             int executed = __popc(in_chunk);
             done = executed < G;
