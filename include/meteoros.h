@@ -171,7 +171,8 @@ typedef struct mt_tuning {
                                * runs on a second stream beside the raymarch (default; the call
                                * still completes in `stream` order); 1 = before it on `stream` */
     int32_t march_block;   /* mt_render: raymarch CTA size, 32, 128 or 256 threads; 0 = default (256);
-                            * launches of one or two lanes per ray take 128 at most */
+                            * launches of one or two lanes per ray take 128 at most, and frames whose
+                            * lengths are out of the ordinary (some 1e7 m and more) the default */
     int32_t march_order;   /* mt_render: 0 = ray rows dispatched bottom to top (default: the rows
                             * below the horizon, which do not march, first, then the marching rows
                             * from the horizon up); 1 = top to bottom */

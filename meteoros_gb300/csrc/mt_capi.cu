@@ -894,9 +894,9 @@ MT_API mt_status mt_render_batch(mt_ctx* ctx, const mt_view* views, int n_views,
     b.tile_h = th;
     b.tame = tame ? 1 : 0;
     const int storage = views[0].params.storage;
-    int blocks = storage == MT_STORAGE_F16    ? mt::batch_blocks_f16(ctx->device, lanes)
-                 : storage == MT_STORAGE_BF16 ? mt::batch_blocks_bf16(ctx->device, lanes)
-                                              : mt::batch_blocks_u8(ctx->device, lanes);
+    int blocks = storage == MT_STORAGE_F16    ? mt::batch_blocks_f16(ctx->device, lanes, tame)
+                 : storage == MT_STORAGE_BF16 ? mt::batch_blocks_bf16(ctx->device, lanes, tame)
+                                              : mt::batch_blocks_u8(ctx->device, lanes, tame);
 
     if (ctx->batch_direct) {
         // The same work as the graph below, issued on the caller's stream.
@@ -1352,9 +1352,9 @@ MT_API mt_status mt_render_batch_noalloc(mt_ctx* ctx, const mt_view* views, int 
     b.tame = tame ? 1 : 0;
     const int storage = views[0].params.storage;
     const int lanes = ctx->batch_lanes;
-    const int blocks = storage == MT_STORAGE_F16    ? mt::batch_blocks_f16(ctx->device, lanes)
-                       : storage == MT_STORAGE_BF16 ? mt::batch_blocks_bf16(ctx->device, lanes)
-                                                    : mt::batch_blocks_u8(ctx->device, lanes);
+    const int blocks = storage == MT_STORAGE_F16    ? mt::batch_blocks_f16(ctx->device, lanes, tame)
+                       : storage == MT_STORAGE_BF16 ? mt::batch_blocks_bf16(ctx->device, lanes, tame)
+                                                    : mt::batch_blocks_u8(ctx->device, lanes, tame);
     MT_CUDA(ctx, storage == MT_STORAGE_F16    ? mt::launch_batch_f16(b, lanes, blocks, s)
                  : storage == MT_STORAGE_BF16 ? mt::launch_batch_bf16(b, lanes, blocks, s)
                                               : mt::launch_batch_u8(b, lanes, blocks, s));

@@ -228,9 +228,9 @@ cudaError_t launch_batch_u8(const BatchArgs& b, int lanes, int blocks, cudaStrea
 cudaError_t launch_batch_f16(const BatchArgs& b, int lanes, int blocks, cudaStream_t s);
 cudaError_t launch_batch_bf16(const BatchArgs& b, int lanes, int blocks, cudaStream_t s);
 // CTAs of the persistent batched march that fit on the device at once.
-int batch_blocks_u8(int device, int lanes);
-int batch_blocks_f16(int device, int lanes);
-int batch_blocks_bf16(int device, int lanes);
+int batch_blocks_u8(int device, int lanes, bool tame);
+int batch_blocks_f16(int device, int lanes, bool tame);
+int batch_blocks_bf16(int device, int lanes, bool tame);
 cudaError_t launch_march_f16(const MarchArgs& a, cudaStream_t s);
 cudaError_t launch_march_bf16(const MarchArgs& a, cudaStream_t s);
 cudaError_t launch_txaa(const TxaaArgs& a, cudaStream_t s, const cudaEvent_t* ev);

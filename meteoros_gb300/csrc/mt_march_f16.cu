@@ -8,5 +8,7 @@ cudaError_t launch_march_f16(const MarchArgs& a, cudaStream_t s) {
 cudaError_t launch_batch_f16(const BatchArgs& b, int lanes, int blocks, cudaStream_t s) {
     return launch_batch_storage<MT_STORAGE_F16>(b, lanes, blocks, s);
 }
-int batch_blocks_f16(int device, int lanes) { return batch_blocks_storage<MT_STORAGE_F16>(device, lanes); }
+int batch_blocks_f16(int device, int lanes, bool tame) {
+    return batch_blocks_storage<MT_STORAGE_F16>(device, lanes, tame);
+}
 }  // namespace mt
