@@ -302,7 +302,7 @@ def bench_batched(ctx, torch, flush, reps: int = 3) -> dict:
             pms = _timed_reps(torch, flush, per_view, reps)
             out["per_view_u8_fp32"] = {"ms": round(pms, 3),
                                        "gsamples_per_s": round(samples / (pms * 1e-3) / 1e9, 3)}
-    ctx.set_tuning(batch_tile=(16, 8), batch_lanes=1, batch_order=0)
+    ctx.set_tuning(batch_tile=(16, 8), batch_lanes=0, batch_order=0)
     return out
 
 

@@ -162,8 +162,9 @@ typedef struct mt_tuning {
                             * 1 = the raymarch, then the reprojection fused with the TXAA resolve */
     int32_t batch_tile_w;  /* mt_render_batch: tile of rays a CTA takes at a time (default 16 x 8) */
     int32_t batch_tile_h;
-    int32_t batch_lanes;   /* mt_render_batch: lanes per ray, 1, 4, 8 or 16 (default 1; a batch with too
-                            * few rays to fill the GPU at 1 takes more, on smaller tiles) */
+    int32_t batch_lanes;   /* mt_render_batch: lanes per ray, 1, 4, 8 or 16; 0 = chosen from the batch's
+                            * rays (default: 1, or where the rays are too few to fill the GPU at 1
+                            * more, on smaller tiles; mt_render_batch_noalloc: 1) */
     int32_t batch_direct;  /* mt_render_batch: 0 = one CUDA graph per batch (default); 1 = the same
                             * copies and launches issued directly on the stream (no capture
                             * cost per batch: the serving loop's small batches) */

@@ -1,4 +1,4 @@
-// Host rules of a batch that need no CUDA headers.
+// Launch rules of the host that need no CUDA headers.
 #pragma once
 
 #include <algorithm>
@@ -7,6 +7,45 @@
 #include <vector>
 
 namespace mt {
+
+// Lanes that march one ray together when the tuning leaves it open, by the rays
+// of the launch.  More lanes shorten a ray's serial chain (alone some 220 us at
+// one lane, 25 at 32) and fill the 152 SMs' 155 648 resident threads; they also
+// compute steps past a ray's exit and scan.  Measured both sides of each line,
+// us by view (frames are checkerboard, 1/16 of the pixels):
+//   32 | 16  480x270 frame 46 / 36 | 42 / 41, 128x72 full 36 / 25 | 30 / 30
+//   16 | 8   800x450 frame 65 / 53 | 69 / 65, 960x540 frame 82 / 65 | 77 / 70
+//   8 | 4    1440x810 frame 136 / 114 | 141 / 163, 1600x900 frame 164 / 136 | 161 / 159
+//   4 | 2    2240x1260 frame 270 / 220 | 251 / 263, 2560x1440 frame 346 / 282 | 307 / 267
+//   2 | 1    3000x1688 frame 417 / 347 | 407 / 466, 860x484 full 311 / 200 | 294 / 219,
+//            960x540 full 371 / 241 | 345 / 230
+inline int auto_lanes(long long rays) {
+    if (rays <= 8192) return 32;
+    if (rays <= 28000) return 16;
+    if (rays <= 90000) return 8;
+    if (rays <= 210000) return 4;
+    return rays <= 450000 ? 2 : 1;
+}
+
+struct BatchShape {
+    int lanes, tile_w, tile_h;
+};
+
+// The lanes and tile of a batch of `rays`: those asked for, or with 0 lanes what
+// mt_render would take, on tiles shrunk to one pass each (a CTA's 128 threads)
+// where the rays are too few to fill the GPU at one lane: two sessions' frames
+// (72 000 rays) 307 / 398 -> 168 / 192 us by view.
+inline BatchShape batch_shape(int lanes, int tile_w, int tile_h, long long rays) {
+    if (lanes != 0) return BatchShape{lanes, tile_w, tile_h};
+    lanes = auto_lanes(rays);
+    while (lanes > 1 && tile_w * tile_h > 128 / lanes) {
+        if (tile_w >= tile_h)
+            tile_w = (tile_w + 1) / 2;
+        else
+            tile_h = (tile_h + 1) / 2;
+    }
+    return BatchShape{lanes, tile_w, tile_h};
+}
 
 // The bytes of an image that a batch's reprojections read or write.
 struct ImageBytes {

@@ -61,7 +61,7 @@ struct mt_ctx {
     uint8_t* tga_dev = nullptr;
     size_t tga_bytes = 0;
     // mt_render_batch
-    int batch_tile_w = 16, batch_tile_h = 8, batch_lanes = 1;
+    int batch_tile_w = 16, batch_tile_h = 8, batch_lanes = 0;  // 0: by the rays
     int batch_direct = 0;                     // 1: no graph, copies and launches issued on the stream
     // Two slots used in turn, so two batches may run at once on two streams.
     mt::MarchArgs* d_views[2] = {nullptr, nullptr};  // device view tables
@@ -775,23 +775,6 @@ mt_status ensure_batch_buffers(mt_ctx* ctx, size_t n_views, size_t n_tiles) {
     return MT_OK;
 }
 
-// The lanes and tile of a batch of `rays`: the tuning's, except that one lane
-// per ray becomes what mt_render would take where the rays are too few to fill
-// the GPU, on tiles of one pass each (a CTA's 128 threads): two sessions' frames
-// (72 000 rays) 307 / 398 -> 168 / 192 us by view.
-void batch_shape(const mt_ctx* ctx, long long rays, int* lanes, int* tw, int* th) {
-    *tw = ctx->batch_tile_w;
-    *th = ctx->batch_tile_h;
-    *lanes = ctx->batch_lanes == 1 ? mt::auto_lanes(rays) : ctx->batch_lanes;
-    if (ctx->batch_lanes != 1 || *lanes == 1) return;
-    while (*tw * *th > 128 / *lanes) {
-        if (*tw >= *th)
-            *tw = (*tw + 1) / 2;
-        else
-            *th = (*th + 1) / 2;
-    }
-}
-
 // The graph branches a batch's reprojections may spread over: one, in view order,
 // where a view's frame is another's previous frame or the same image (a recycled
 // image is read before it is written, as when the views are rendered one by one).
@@ -852,8 +835,8 @@ MT_API mt_status mt_render_batch(mt_ctx* ctx, const mt_view* views, int n_views,
         ray_grid(a, &nx, &ny);
         rays += (long long)nx * ny;
     }
-    int lanes, tw, th;
-    batch_shape(ctx, rays, &lanes, &tw, &th);
+    const mt::BatchShape shape = mt::batch_shape(ctx->batch_lanes, ctx->batch_tile_w, ctx->batch_tile_h, rays);
+    const int lanes = shape.lanes, tw = shape.tile_w, th = shape.tile_h;
     std::vector<int> order((size_t)n_views);
     for (int i = 0; i < n_views; ++i) order[(size_t)i] = i;
     auto cost = [&](int i) {
@@ -1072,8 +1055,9 @@ MT_API mt_status mt_set_tuning(mt_ctx* ctx, const mt_tuning* t) {
         return fail(ctx, MT_ERR_INVALID_ARG, "fused_resolve must be 0 or 1");
     if (t->batch_tile_w < 1 || t->batch_tile_h < 1 || t->batch_tile_w * t->batch_tile_h > 4096)
         return fail(ctx, MT_ERR_INVALID_ARG, "batch tile must be 1..4096 rays");
-    if (t->batch_lanes != 1 && t->batch_lanes != 4 && t->batch_lanes != 8 && t->batch_lanes != 16)
-        return fail(ctx, MT_ERR_INVALID_ARG, "batch_lanes must be 1, 4, 8 or 16");
+    if (t->batch_lanes != 0 && t->batch_lanes != 1 && t->batch_lanes != 4 && t->batch_lanes != 8 &&
+        t->batch_lanes != 16)
+        return fail(ctx, MT_ERR_INVALID_ARG, "batch_lanes must be 0 (auto), 1, 4, 8 or 16");
     if (t->batch_direct != 0 && t->batch_direct != 1) return fail(ctx, MT_ERR_INVALID_ARG, "batch_direct must be 0 or 1");
     if (t->reproject_serial != 0 && t->reproject_serial != 1)
         return fail(ctx, MT_ERR_INVALID_ARG, "reproject_serial must be 0 or 1");
@@ -1351,7 +1335,7 @@ MT_API mt_status mt_render_batch_noalloc(mt_ctx* ctx, const mt_view* views, int 
     b.tile_h = th;
     b.tame = tame ? 1 : 0;
     const int storage = views[0].params.storage;
-    const int lanes = ctx->batch_lanes;
+    const int lanes = ctx->batch_lanes ? ctx->batch_lanes : 1;  // the fixed tile list takes whole tiles
     const int blocks = storage == MT_STORAGE_F16    ? mt::batch_blocks_f16(ctx->device, lanes, tame)
                        : storage == MT_STORAGE_BF16 ? mt::batch_blocks_bf16(ctx->device, lanes, tame)
                                                     : mt::batch_blocks_u8(ctx->device, lanes, tame);

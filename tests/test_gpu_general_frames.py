@@ -29,7 +29,7 @@ def ctx(lib):
 @pytest.fixture(autouse=True)
 def tuning(ctx):
     yield
-    ctx.set_tuning(march_lanes=0, batch_lanes=1, batch_tile=(16, 8), batch_direct=False)
+    ctx.set_tuning(march_lanes=0, batch_lanes=0, batch_tile=(16, 8), batch_direct=False)
 
 
 def counts(st):
