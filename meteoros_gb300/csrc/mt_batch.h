@@ -19,10 +19,17 @@ namespace mt {
 //   4 | 2    2240x1260 frame 270 / 220 | 251 / 263, 2560x1440 frame 346 / 282 | 307 / 267
 //   2 | 1    3000x1688 frame 417 / 347 | 407 / 466, 860x484 full 311 / 200 | 294 / 219,
 //            960x540 full 371 / 241 | 345 / 230
-inline int auto_lanes(long long rays) {
-    if (rays <= 8192) return 32;
-    if (rays <= 28000) return 16;
-    if (rays <= 90000) return 8;
+// The lines above are RGBA8's.  On 16-bit volumes a step costs more (wider texels to
+// load and convert), and steps past the exit with it: the three upper lines lie
+// lower (FP16 full frames, us by view; bfloat16's cross at the same places):
+//   32 | 16  75x73 53 / 47 / 46 | 48 / 48 / 47, 89x89 62 / 64 / 56 | 54 / 52 / 48
+//   16 | 8   130x130 71 / 79 / 65 | 74 / 73 / 69, 180x155 103 / 107 / 90 | 82 / 82 / 79
+//   8 | 4    255x255 142 / 141 / 113 | 142 / 135 / 135, 300x300 176 / 180 / 142 | 153 / 141 / 133
+//   2 | 1    550x550 324 / 271 / 226 | 358 / 359 / 337, 670x670 437 / 355 / 277 | 418 / 404 / 365
+inline int auto_lanes(long long rays, bool texels16) {
+    if (rays <= (texels16 ? 5500 : 8192)) return 32;
+    if (rays <= (texels16 ? 17000 : 28000)) return 16;
+    if (rays <= (texels16 ? 66000 : 90000)) return 8;
     if (rays <= 210000) return 4;
     return rays <= 450000 ? 2 : 1;
 }
@@ -31,13 +38,13 @@ struct BatchShape {
     int lanes, tile_w, tile_h;
 };
 
-// The lanes and tile of a batch of `rays`: those asked for, or with 0 lanes what
-// mt_render would take, on tiles shrunk to one pass each (a CTA's 128 threads)
+// The lanes and tile of a batch: those asked for, or with 0 lanes what mt_render
+// would take for its rays (`by_rays`), on tiles shrunk to one pass each (a CTA's 128 threads)
 // where the rays are too few to fill the GPU at one lane: two sessions' frames
 // (72 000 rays) 307 / 398 -> 168 / 192 us by view.
-inline BatchShape batch_shape(int lanes, int tile_w, int tile_h, long long rays) {
+inline BatchShape batch_shape(int lanes, int tile_w, int tile_h, int by_rays) {
     if (lanes != 0) return BatchShape{lanes, tile_w, tile_h};
-    lanes = auto_lanes(rays);
+    lanes = by_rays;
     while (lanes > 1 && tile_w * tile_h > 128 / lanes) {
         if (tile_w >= tile_h)
             tile_w = (tile_w + 1) / 2;

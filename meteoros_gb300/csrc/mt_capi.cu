@@ -282,7 +282,8 @@ mt_status build_march_args(mt_ctx* ctx, const mt_camera_ubo* cam, const mt_camer
     a->bottom_up = ctx->march_order == 0 ? 1 : 0;
     a->lanes = ctx->march_lanes;
     // (a checkerboard frame marches a sixteenth of its pixels)
-    if (a->lanes == 0) a->lanes = mt::auto_lanes((long long)w * h / (full ? 1 : 16));
+    if (a->lanes == 0)
+        a->lanes = mt::auto_lanes((long long)w * h / (full ? 1 : 16), p->storage != MT_STORAGE_U8);
     return MT_OK;
 }
 
@@ -835,7 +836,9 @@ MT_API mt_status mt_render_batch(mt_ctx* ctx, const mt_view* views, int n_views,
         ray_grid(a, &nx, &ny);
         rays += (long long)nx * ny;
     }
-    const mt::BatchShape shape = mt::batch_shape(ctx->batch_lanes, ctx->batch_tile_w, ctx->batch_tile_h, rays);
+    const int storage = views[0].params.storage;
+    const mt::BatchShape shape = mt::batch_shape(ctx->batch_lanes, ctx->batch_tile_w, ctx->batch_tile_h,
+                                                 mt::auto_lanes(rays, storage != MT_STORAGE_U8));
     const int lanes = shape.lanes, tw = shape.tile_w, th = shape.tile_h;
     std::vector<int> order((size_t)n_views);
     for (int i = 0; i < n_views; ++i) order[(size_t)i] = i;
@@ -876,7 +879,6 @@ MT_API mt_status mt_render_batch(mt_ctx* ctx, const mt_view* views, int n_views,
     b.tile_w = tw;
     b.tile_h = th;
     b.tame = tame ? 1 : 0;
-    const int storage = views[0].params.storage;
     int blocks = storage == MT_STORAGE_F16    ? mt::batch_blocks_f16(ctx->device, lanes, tame)
                  : storage == MT_STORAGE_BF16 ? mt::batch_blocks_bf16(ctx->device, lanes, tame)
                                               : mt::batch_blocks_u8(ctx->device, lanes, tame);
