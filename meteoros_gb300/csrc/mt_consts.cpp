@@ -100,9 +100,10 @@ namespace {
 // is six checks, a tenth of an empty step's instructions, and this settles
 // them once per frame (1080p frame 227 / 186 -> 221 / 182 us by view, 4K full
 // frames 5.36 / 3.55 -> 5.12 / 3.39 ms, 20-view batch 11.3 / 9.37 -> 10.9 / 8.97 ms):
-//   * no quotient is large: the scene's lengths are at most kFar, so positions
-//     (t at most the outer shell hit's distance, to the rounding of a quadratic
-//     in |eye| / radius) stay below 2^50 and quotients below 2^80;
+//   * no quotient is large: t, the outer shell hit's distance from the origin, stays
+//     below kMaxT (with a tenth for the rounding of a quadratic in |eye| / radius),
+//     the eye within kFar of the origin and denominators above kScale, so positions
+//     stay below 2^31 and quotients below 2^62;
 //   * a small quotient changes nothing.  Zero is exact up to its sign.  A
 //     texture coordinate below 2^-99 leaves s * N - 0.5 at -0.5.  The components
 //     of the up vector enter dot(dir, up) = (dx ux + dy uy) + dz uz, where dy is
@@ -114,23 +115,24 @@ namespace {
 // and clamps (kExact, mt_march.cuh).  Other frames are marched with the checks
 // (kGeneral).
 bool frame_is_tame(const Frame& f, const mt_params& p, const float jitter[16][3]) {
-    const double kFar = 0x1p30, kSmall = 0x1p-10, kScale = 0x1p-20;
+    const double kFar = 0x1p30, kSmall = 0x1p-10, kScale = 0x1p-20, kMaxT = 0x1p24 - 16.0;
     auto len = [](const float v[3]) {
         return std::sqrt((double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2]);
     };
-    bool ok = len(f.eye) <= kFar && len(f.ec) <= kFar && f.Rout <= kFar && f.R >= kSmall && f.Rin >= kSmall &&
-              f.thickness >= kSmall && p.noise_period >= kScale && p.noise_period <= kFar &&
-              len(f.wind_t) <= kFar && len(f.skew) * std::fabs(p.cloud_top_offset) <= kFar &&
+    bool ok = len(f.eye) <= kFar && f.R >= kSmall && f.Rin >= kSmall && f.thickness >= kSmall &&
+              p.noise_period >= kScale && p.noise_period <= kFar && len(f.wind_t) <= kFar &&
+              len(f.skew) * std::fabs(p.cloud_top_offset) <= kFar &&
               f.eye[1] >= -0.5f * f.R;
     if (p.coverage_mode == 1) ok = ok && p.weather_scale >= kScale && p.weather_scale <= kFar;
     for (int i = 0; i < 16; ++i)
         for (int c = 0; c < 3; ++c) ok = ok && std::fabs(jitter[i][c]) <= 0.05f;
     // a constant coverage, and its remap's width, 0 or within 2^30 of 1 (a weather
-    // map's are 0 or at least 2^-32); t below 2^24 - 16
+    // map's are 0 or at least 2^-32)
     if (p.coverage_mode == 0)
         for (const double c : {std::fabs((double)p.coverage), std::fabs((double)(1.0f - p.coverage))})
             ok = ok && (c == 0.0 || (c >= 0x1p-30 && c <= 0x1p30));
-    ok = ok && 1.1 * (len(f.ec) + f.Rout + std::fmax(len(f.sh32_o[0]), len(f.sh32_o[1]))) < 0x1p24 - 16.0;
+    // the Earth's centre and its outer shell too: bounds the planet and the eye's x and z
+    ok = ok && 1.1 * (len(f.ec) + f.Rout + std::fmax(len(f.sh32_o[0]), len(f.sh32_o[1]))) < kMaxT;
     return ok;  // false for NaN
 }
 
