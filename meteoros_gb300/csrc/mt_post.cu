@@ -254,6 +254,7 @@ __global__ void __launch_bounds__(32 * kGodWarps) godrays_kernel(const __grid_co
         __syncthreads();
     }
     const GodrayFrame g = ROWS > 1 ? frame : godray_frame(a.camera);
+    const bool blurs = !(g.blend < 0.0f) && !g.outside;  // else the image passes as it is, and needs no taps
     const GodAxis col = god_axis(px, W, g.ssx);
     // one row a thread: its own; else the row that this thread tabulates
     GodAxis row = god_axis(y0 + (ROWS == 1 ? first : (int)threadIdx.x & (TH - 1)), H, g.ssy);
@@ -265,13 +266,13 @@ __global__ void __launch_bounds__(32 * kGodWarps) godrays_kernel(const __grid_co
             pixel_y[threadIdx.x] = row.pixel;
             covered_y[threadIdx.x] = row.covered;
 #pragma unroll 10
-            for (int i = 0; i < kGodTaps; ++i) {
+            for (int i = 0; blurs && i < kGodTaps; ++i) {
                 taps[i * TH + threadIdx.x].w = row.u;
                 row.u -= row.d;
             }
         }
         __syncthreads();
-        for (int e = (int)threadIdx.x; e < kGodTaps * TH; e += 32 * kGodWarps) {  // whole warps
+        for (int e = (int)threadIdx.x; blurs && e < kGodTaps * TH; e += 32 * kGodWarps) {  // whole warps
             const AxisTap y = axis_tap(taps[e].w, (float)H);
             const int below = __shfl_down_sync(0xffffffffu, y.i, 1, TH);
             chain = chain && (e < TH || (unsigned)below - (unsigned)y.i <= 1u);
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(32 * kGodWarps) godrays_kernel(const __grid_co
     float2 ax[PAIRS], ay[PAIRS], az[PAIRS];
 #pragma unroll
     for (int k = 0; k < PAIRS; ++k) ax[k] = ay[k] = az[k] = make_float2(0.0f, 0.0f);
-    if (!(g.blend < 0.0f) && !g.outside) {
+    if (blurs) {
         if (inside && a.light[0] == a.light[1])
             god_blur<ROWS, true, true>(a, taps + first, col, row, ax, ay, az);
         else if (inside)
