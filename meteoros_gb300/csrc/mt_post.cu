@@ -64,9 +64,11 @@ MT_HD AxisTap axis_tap(float u, float n) {
 // to bitDec.w.  LINEAR filter with exact FP32 weights, like every sampler
 // here: the value channel and the border channel are interpolated x then y,
 // then decoded as dot(texel, bitDec) in the shader's order.  INSIDE: all four
-// texels are in the image, where the border channel is 0.
-template <bool INSIDE> MT_HD float mask_decode(const GodrayArgs& a, AxisTap x, AxisTap y) {
-    if (INSIDE || ((unsigned)x.i < (unsigned)(a.width - 1) && (unsigned)y.i < (unsigned)(a.height - 1))) {
+// texels are in the image, where the border channel is 0.  FLAT: no branch at the
+// border, the texels' indices clamped instead, so that several taps' loads are in
+// flight together.
+template <bool INSIDE, bool FLAT> MT_HD float mask_decode(const GodrayArgs& a, AxisTap x, AxisTap y) {
+    if (INSIDE || (!FLAT && (unsigned)x.i < (unsigned)(a.width - 1) && (unsigned)y.i < (unsigned)(a.height - 1))) {
         const float* r = a.mask + (y.i * a.width + x.i);
         const float* r1 = r + a.width;
         const float2 p = make_float2(__ldg(r), __ldg(r1)), q = make_float2(__ldg(r + 1), __ldg(r1 + 1));
@@ -77,8 +79,10 @@ template <bool INSIDE> MT_HD float mask_decode(const GodrayArgs& a, AxisTap x, A
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int i = x.i + (k & 1), j = y.i + (k >> 1);
+        const int ic = FLAT ? imin(imax(i, 0), a.width - 1) : i, jc = FLAT ? imin(imax(j, 0), a.height - 1) : j;
         const bool out = i < 0 || j < 0 || i >= a.width || j >= a.height;
-        val[k] = out ? 0.0f : __ldg(a.mask + (size_t)j * (size_t)a.width + (size_t)i);
+        const float t = FLAT || !out ? __ldg(a.mask + (jc * a.width + ic)) : 0.0f;
+        val[k] = out ? 0.0f : t;
         brd[k] = out ? 1.0f : 0.0f;
     }
     const float v = lerp1(lerp1(val[0], val[1], x.w), lerp1(val[2], val[3], x.w), y.w);
@@ -141,6 +145,11 @@ constexpr int kGodTaps = 100, kGodWarps = 4;
 // (1 | 2 | 4 rows, us: 320x180 25 | 42 | -, 640x360 54 | 44 | -, 1280x720 141 | 121 | -,
 // 1920x1080 283 | 229 | 222; 8 rows 268).
 constexpr long long kRows2 = 200000, kRows4 = 1800000;
+// Small images are latency: up to here the taps take no branch at the border and are
+// unrolled by 20 (branch, by 4 | flat, us, sun in the image and at its edge: 160x90
+// 25 / 33 | 17 / 17, 256x144 25 / 35 | 19 / 19, 320x180 25 / 39 | 25 / 23, 400x225 28 / 41 |
+// 33 / 33, 640x360 43 / 64 | 62 / 64).
+constexpr long long kFlat = 72000;
 
 // One axis of a fragment: its first tap, its step and whether all its taps keep a
 // texel and a half from the ends (the recurrence's roundings move a tap by less
@@ -171,13 +180,19 @@ MT_HD GodAxis god_axis(int f, int n, float ss) {
 // close in on the sun together.  Then the rows' filtered texels chain: a row's
 // upper texels are its upper neighbour's, upper or lower, and it loads and filters
 // its lower two, in packed pairs of rows.
-template <int ROWS, bool INSIDE, bool SHARED_RG>
+template <int ROWS, bool INSIDE, bool FLAT, bool SHARED_RG>
 MT_HD void god_blur(const GodrayArgs& a, const AxisTap* rows, GodAxis col, GodAxis row, float2 (&ax)[(ROWS + 1) / 2],
                     float2 (&ay)[(ROWS + 1) / 2], float2 (&az)[(ROWS + 1) / 2]) {
     constexpr int TH = kGodWarps * ROWS, PAIRS = (ROWS + 1) / 2;
     const float w = 1.0f * 0.001f;  // illuminationDecay * WEIGHT_FOR_SAMPLE, DECAY = 1
     const float fw = (float)a.width, fh = (float)a.height;
     auto add = [&](int k, float2 s) {
+        if (ROWS == 1) {  // no pair to fill
+            ax[0].x = ax[0].x + (a.light[0] * s.x) * w;
+            if (!SHARED_RG) ay[0].x = ay[0].x + (a.light[1] * s.x) * w;
+            az[0].x = az[0].x + (a.light[2] * s.x) * w;
+            return;
+        }
         auto weighted = [&](float light) { return mul2(mul2(splat2(light), s), splat2(w)); };
         ax[k] = add2(ax[k], weighted(a.light[0]));
         if (!SHARED_RG) ay[k] = add2(ay[k], weighted(a.light[1]));
@@ -191,7 +206,7 @@ MT_HD void god_blur(const GodrayArgs& a, const AxisTap* rows, GodAxis col, GodAx
 #pragma unroll
             for (int h = 0; h < 2 && 2 * k + h < ROWS; ++h) {
                 const AxisTap y = ROWS == 1 ? axis_tap(row.u, fh) : rows[i * TH + 2 * k + h];
-                s[h] = mask_decode<INSIDE>(a, x, y);
+                s[h] = mask_decode<INSIDE, FLAT>(a, x, y);
             }
             add(k, make_float2(s[0], s[1]));
         }
@@ -229,7 +244,7 @@ MT_HD void god_blur(const GodrayArgs& a, const AxisTap* rows, GodAxis col, GodAx
             col.u -= col.d;
         }
     } else {
-        constexpr int kUnroll = ROWS == 1 ? 4 : 2;
+        constexpr int kUnroll = FLAT ? 20 : ROWS == 1 ? 4 : 2;
 #pragma unroll kUnroll
         for (int i = 0; i < kGodTaps; ++i) single(i);
     }
@@ -239,7 +254,7 @@ MT_HD void god_blur(const GodrayArgs& a, const AxisTap* rows, GodAxis col, GodAx
     }
 }
 
-template <int ROWS>
+template <int ROWS, bool FLAT>
 __global__ void __launch_bounds__(32 * kGodWarps) godrays_kernel(const __grid_constant__ GodrayArgs a) {
     constexpr int TH = kGodWarps * ROWS;
     __shared__ __align__(16) AxisTap taps[ROWS == 1 ? 1 : kGodTaps * TH];
@@ -286,11 +301,11 @@ __global__ void __launch_bounds__(32 * kGodWarps) godrays_kernel(const __grid_co
     for (int k = 0; k < PAIRS; ++k) ax[k] = ay[k] = az[k] = make_float2(0.0f, 0.0f);
     if (blurs) {
         if (inside && a.light[0] == a.light[1])
-            god_blur<ROWS, true, true>(a, taps + first, col, row, ax, ay, az);
+            god_blur<ROWS, true, FLAT, true>(a, taps + first, col, row, ax, ay, az);
         else if (inside)
-            god_blur<ROWS, true, false>(a, taps + first, col, row, ax, ay, az);
+            god_blur<ROWS, true, FLAT, false>(a, taps + first, col, row, ax, ay, az);
         else
-            god_blur<ROWS, false, false>(a, taps + first, col, row, ax, ay, az);
+            god_blur<ROWS, false, FLAT, false>(a, taps + first, col, row, ax, ay, az);
     }
     if (px >= W) return;
 #pragma unroll
@@ -411,11 +426,13 @@ cudaError_t launch_godrays(const GodrayArgs& a, cudaStream_t s) {
     const unsigned gx = (unsigned)((a.width + 31) / 32);
     const long long pixels = (long long)a.width * a.height;
     if (pixels >= kRows4)
-        godrays_kernel<4><<<dim3(gx, (unsigned)((a.height + 15) / 16)), 128, 0, s>>>(a);
+        godrays_kernel<4, false><<<dim3(gx, (unsigned)((a.height + 15) / 16)), 128, 0, s>>>(a);
     else if (pixels >= kRows2)
-        godrays_kernel<2><<<dim3(gx, (unsigned)((a.height + 7) / 8)), 128, 0, s>>>(a);
+        godrays_kernel<2, false><<<dim3(gx, (unsigned)((a.height + 7) / 8)), 128, 0, s>>>(a);
+    else if (pixels > kFlat)
+        godrays_kernel<1, false><<<dim3(gx, (unsigned)((a.height + 3) / 4)), 128, 0, s>>>(a);
     else
-        godrays_kernel<1><<<dim3(gx, (unsigned)((a.height + 3) / 4)), 128, 0, s>>>(a);
+        godrays_kernel<1, true><<<dim3(gx, (unsigned)((a.height + 3) / 4)), 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 
