@@ -276,10 +276,11 @@ __device__ __forceinline__ void flush_counts(unsigned long long* stats, const Co
     unsigned rays = __reduce_add_sync(0xffffffffu, c.rays);
     unsigned pix = __reduce_add_sync(0xffffffffu, pixels);
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(stats + 0, (unsigned long long)prim);
-        atomicAdd(stats + 1, (unsigned long long)light);
-        atomicAdd(stats + 2, (unsigned long long)rays);
-        atomicAdd(stats + 3, (unsigned long long)pix);
+        // every warp adds to the same four words: no additions of 0
+        if (prim) atomicAdd(stats + 0, (unsigned long long)prim);
+        if (light) atomicAdd(stats + 1, (unsigned long long)light);
+        if (rays) atomicAdd(stats + 2, (unsigned long long)rays);
+        if (pix) atomicAdd(stats + 3, (unsigned long long)pix);
     }
 }
 
