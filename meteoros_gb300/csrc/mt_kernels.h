@@ -150,7 +150,6 @@ struct BatchArgs {
     int32_t tame;               // every view's frame is (Frame::tame)
 };
 
-// Outputs of one generator launch (any pointer may be NULL).
 // postProcess_GodRays.frag over an HDR image (mt_godrays)
 struct GodrayArgs {
     mt_camera_ubo camera;
@@ -177,6 +176,7 @@ struct TgaSlice {
     long long size;
 };
 
+// Outputs of the generator: a volume's texels in their three storages.
 struct NoiseOut {
     uint32_t* u8;   // RGBA8 words
     uint2* h16;     // 4 x IEEE half per texel

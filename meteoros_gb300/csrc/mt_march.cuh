@@ -234,7 +234,7 @@ MT_HD StepOut eval_step(const mt_params& p, const Frame& F, const Tex<S>& tx, co
     Weather wt = weather_at<S, TAME>(p, F, tx, pos, ld3(F.ec));
     // (the 16-bit forms keep its check: without it their compiler settings
     // contract its blends another way, which moves their results by roundings)
-    if (p.height_gradient) wt.hgrad = height_gradient<EXACT, EXACT>(relH, wt.type);
+    if (p.height_gradient) wt.hgrad = height_gradient<EXACT>(relH, wt.type);
     // ... a zero height gradient or zero coverage makes the density 0 (or NaN
     // when the coverage is 0), never > 0 ...
     if ((p.height_gradient && wt.hgrad == 0.0f) || wt.mul == 0.0f) return o;

@@ -148,12 +148,13 @@ static __device__ __noinline__ HgQuot hg_quotients_exceptional(float h) {
 // cloudRayMarch.comp:475-487.  The remaps' four quotients share one range
 // check (rdiv_core; all four redone by rdiv when any falls outside it).
 // EXACT: the same values from saturating and min/max instructions, which differ
-// from the shader's selects in the sign of a zero only (no operand is NaN).
-template <bool TAME, bool EXACT> MT_HD float height_gradient(float h, float type) {
+// from the shader's selects in the sign of a zero only (no operand is NaN),
+// and take no range check.
+template <bool EXACT> MT_HD float height_gradient(float h, float type) {
     h = EXACT ? __saturatef(h) : gclamp(h, 0.0f, 1.0f);
     HgQuot q{rdiv_core(h - 0.0f, MT_RCP(0.0f, 0.25f)), rdiv_core(h - 0.3f, MT_RCP(0.3f, 0.65f)),
              rdiv_core(h - 0.0f, MT_RCP(0.0f, 0.1f)), rdiv_core(h - 0.2f, MT_RCP(0.2f, 0.3f))};
-    if (!TAME && !(rdiv_in_range(q.q1) & rdiv_in_range(q.q2) & rdiv_in_range(q.q3) & rdiv_in_range(q.q4)))
+    if (!EXACT && !(rdiv_in_range(q.q1) & rdiv_in_range(q.q2) & rdiv_in_range(q.q3) & rdiv_in_range(q.q4)))
         q = hg_quotients_exceptional(h);
     // remap(h, omin, omax, nmin, nmax) = nmin + q * (nmax - nmin)
     if (EXACT) {
