@@ -9,8 +9,8 @@
 namespace mt {
 
 // Lanes that march one ray together when the tuning leaves it open, by the rays
-// of the launch.  More lanes shorten a ray's serial chain (alone some 220 us at
-// one lane, 25 at 32) and fill the 152 SMs' 155 648 resident threads; they also
+// of the launch.  More lanes shorten a ray's serial chain (32 rays alone take 159
+// to 218 us by view at one lane, 18 to 20 at 32) and fill the 152 SMs' 155 648 resident threads; they also
 // compute steps past a ray's exit and scan.  Measured both sides of each line,
 // us by view (frames are checkerboard, 1/16 of the pixels):
 //   32 | 16  480x270 frame 46 / 36 | 42 / 41, 128x72 full 36 / 25 | 30 / 30
@@ -25,7 +25,7 @@ namespace mt {
 //   32 | 16  75x73 53 / 47 / 46 | 48 / 48 / 47, 89x89 62 / 64 / 56 | 54 / 52 / 48
 //   16 | 8   130x130 71 / 79 / 65 | 74 / 73 / 69, 180x155 103 / 107 / 90 | 82 / 82 / 79
 //   8 | 4    255x255 142 / 141 / 113 | 142 / 135 / 135, 300x300 176 / 180 / 142 | 153 / 141 / 133
-//   2 | 1    550x550 324 / 271 / 226 | 358 / 359 / 337, 670x670 437 / 355 / 277 | 418 / 404 / 365
+//   2 | 1    600x600 367 / 304 / 238 | 331 / 321 / 297, 670x670 437 / 355 / 276 | 366 / 347 / 314
 inline int auto_lanes(long long rays, bool texels16) {
     if (rays <= (texels16 ? 5500 : 8192)) return 32;
     if (rays <= (texels16 ? 17000 : 28000)) return 16;
@@ -39,9 +39,9 @@ struct BatchShape {
 };
 
 // The lanes and tile of a batch: those asked for, or with 0 lanes what mt_render
-// would take for its rays (`by_rays`), on tiles shrunk to one pass each (a CTA's 128 threads)
-// where the rays are too few to fill the GPU at one lane: two sessions' frames
-// (72 000 rays) 307 / 398 -> 168 / 192 us by view.
+// would take for its rays (`by_rays`), on tiles shrunk to one pass each (a CTA's
+// 128 threads) where the rays are too few to fill the GPU at one lane: two
+// sessions' frames (72 000 rays) 307 / 398 -> 168 / 192 us by view.
 inline BatchShape batch_shape(int lanes, int tile_w, int tile_h, int by_rays) {
     if (lanes != 0) return BatchShape{lanes, tile_w, tile_h};
     lanes = by_rays;

@@ -497,17 +497,17 @@ MT_HD void march_pixel(const MarchArgs& a, const Frame& F, const Tex<S>& tx, int
 // aligned segment of a warp) march one ray.  BS threads per CTA (256 by
 // default, 128 or 32 selectable; 128 at most for one and two lanes per ray, whose
 // rays end furthest apart: 960x540 full frames 357 / 234 -> 344 / 230 us by view, FP16
-// 4K 3.76 / 2.58 -> 3.70 / 2.54 ms, 640x360 full frame 205 / 140 -> 196 / 139).  Resident threads per SM: 1024 (64 registers
-// a thread), or for one lane per ray on FP16 volumes 1280 (48, with some 200 B
-// of spills: 4K 4.12 ms for 4.19; RGBA8 took 4.69 ms so for 4.62, and bfloat16
-// 1603x901 1.06 ms for 1.01).
+// 4K 3.76 / 2.58 -> 3.70 / 2.54 ms, 640x360 full frame 205 / 140 -> 196 / 139).
+// Resident threads per SM: 1024, 64 registers a thread.  (1280 for one lane per ray,
+// at 48 registers with some 200 B of spills: RGBA8 4K 4.69 ms for 4.62, bfloat16
+// 1603x901 1.06 for 1.01; FP16, us by view, 680x680 417 / 403 / 365 for 375 / 348 /
+// 317, 4K 4775 / 3748 / 3241 for 4641 / 3647 / 3138.)
 // Every step reads its jitter vector at an index taken from int(t), which
 // differs from lane to lane: from the parameter space a warp's reads at up to
 // 16 different words are served one word at a time, from shared memory in one
 // pass (48 words, 3 apart: distinct banks), so the table is copied there.
-constexpr int march_min_blocks(int G, int S, int BS) {
-    const int n = (G == 1 && S == MT_STORAGE_F16 ? 1280 : 1024) / BS;
-    return n < 32 ? n : 32;  // at most 32 CTAs an SM
+constexpr int march_min_blocks(int BS) {
+    return 1024 / BS < 32 ? 1024 / BS : 32;  // at most 32 CTAs an SM
 }
 // The rays of a warp.  One lane per ray: 8x4 rays, which fetch nearer cells and end
 // nearer one another than 32 in a row (960x540 full frames 387 / 235 -> 357 / 234 us by
@@ -524,7 +524,7 @@ template <int G> struct WarpTile {
     }
 };
 template <int G, int S, int BS, int MODE>
-__global__ void __launch_bounds__(BS, march_min_blocks(G, S, BS))
+__global__ void __launch_bounds__(BS, march_min_blocks(BS))
     march_kernel(const __grid_constant__ MarchArgs a) {
     static_assert(G >= 1 && G <= 32 && (32 % G) == 0, "G must divide the warp");
     const Frame& F = a.frame;
