@@ -10,9 +10,9 @@ namespace mt {
 
 // Lanes that march one ray together when the tuning leaves it open, by the rays
 // of the launch.  More lanes shorten a ray's serial chain (32 rays alone take 159
-// to 218 us by view at one lane, 18 to 20 at 32) and fill the 152 SMs' 155 648 resident threads; they also
-// compute steps past a ray's exit and scan.  Measured both sides of each line,
-// us by view (frames are checkerboard, 1/16 of the pixels):
+// to 218 us by view at one lane, 18 to 20 at 32) and fill the 152 SMs' 155 648
+// resident threads; they also compute steps past a ray's exit and scan.  Measured
+// both sides of each line, us by view (frames are checkerboard, 1/16 of the pixels):
 //   32 | 16  480x270 frame 46 / 36 | 42 / 41, 128x72 full 36 / 25 | 30 / 30
 //   16 | 8   800x450 frame 65 / 53 | 69 / 65, 960x540 frame 82 / 65 | 77 / 70
 //   8 | 4    1440x810 frame 136 / 114 | 141 / 163, 1600x900 frame 164 / 136 | 161 / 159
@@ -20,16 +20,21 @@ namespace mt {
 //   2 | 1    3000x1688 frame 417 / 347 | 407 / 466, 860x484 full 311 / 200 | 294 / 219,
 //            960x540 full 371 / 241 | 345 / 230
 // The lines above are RGBA8's.  On 16-bit volumes a step costs more (wider texels to
-// load and convert), and steps past the exit with it: the three upper lines lie
-// lower (FP16 full frames, us by view; bfloat16's cross at the same places):
-//   32 | 16  75x73 53 / 47 / 46 | 48 / 48 / 47, 89x89 62 / 64 / 56 | 54 / 52 / 48
-//   16 | 8   130x130 71 / 79 / 65 | 74 / 73 / 69, 180x155 103 / 107 / 90 | 82 / 82 / 79
-//   8 | 4    255x255 142 / 141 / 113 | 142 / 135 / 135, 300x300 176 / 180 / 142 | 153 / 141 / 133
-//   2 | 1    600x600 367 / 304 / 238 | 331 / 321 / 297, 670x670 437 / 355 / 276 | 366 / 347 / 314
+// load and convert), and steps past the exit with it, so fewer lanes win from fewer
+// rays on, in a light view (few of its steps in cloud) later than in a heavy one:
+// the two upper lines lie where no view loses more than 5 %, below the mean's
+// crossings (FP16, time of the first over the second, mean and range of 14 views;
+// checkerboard frames and bfloat16 within 0.05 of it):
+//   32 | 16  75x73 1.08, 0.95 to 1.43; 90x90 1.24, 1.05 to 1.56
+//   16 | 8   150x140 1.14, 0.95 to 1.51; 165x160 1.27, 1.15 to 1.44
+//   8 | 4    255x255 1.04, 0.84 to 1.23; 300x300 1.20, 1.06 to 1.39, but 1200x1200
+//            frames 1.13, 0.90 to 1.30: RGBA8's line holds
+//   2 | 1    600x600 367 / 304 / 238 | 331 / 321 / 297 us by view, 670x670
+//            437 / 355 / 276 | 366 / 347 / 314: RGBA8's line holds
 inline int auto_lanes(long long rays, bool texels16) {
-    if (rays <= (texels16 ? 5500 : 8192)) return 32;
-    if (rays <= (texels16 ? 17000 : 28000)) return 16;
-    if (rays <= (texels16 ? 66000 : 90000)) return 8;
+    if (rays <= (texels16 ? 7500 : 8192)) return 32;
+    if (rays <= (texels16 ? 22000 : 28000)) return 16;
+    if (rays <= 90000) return 8;
     if (rays <= 210000) return 4;
     return rays <= 450000 ? 2 : 1;
 }
